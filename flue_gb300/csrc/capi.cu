@@ -118,8 +118,20 @@ size_t ws_bytes_for(int op, const Geom& g, int prec) {
     }
 }
 
+// the least workspace an operation accepts (ws_bytes_for is what it uses best)
+size_t ws_min_bytes_for(int op, const Geom& g, int prec) {
+    if (op == FLUE_OP_FMUNU) {
+        PlaneSet ps;
+        ps.np = 1;
+        ps.mu[0] = 0;
+        ps.nu[0] = 1;
+        return energy_ws_min_bytes(g, prec, ps, false);
+    }
+    return ws_bytes_for(op, g, prec);
+}
+
 int check_ws(int op, const FieldRef& F, size_t ws_bytes, const void* ws) {
-    const size_t need = ws_bytes_for(op, F.g, F.prec);
+    const size_t need = ws_min_bytes_for(op, F.g, F.prec);
     if (need && (!ws || ws_bytes < need)) {
         snprintf(g_detail, sizeof(g_detail), "workspace too small: need %zu bytes, got %zu", need, ws_bytes);
         return FLUE_ERR_WORKSPACE;
@@ -158,7 +170,7 @@ int energy_common(const flue_field* U, const PlaneSet& ps, int op, double* d_E, 
     if (rc) return rc;
     if (form != FLUE_FORCE_LIE && form != FLUE_FORCE_EUCLID) return fail(FLUE_ERR_ARG, "bad force form");
     if (!d_E && !d_force) return fail(FLUE_ERR_ARG, "nothing to compute");
-    const size_t need = energy_ws_bytes(F.g, F.prec, ps, d_force != nullptr);
+    const size_t need = energy_ws_min_bytes(F.g, F.prec, ps, d_force != nullptr);
     if (!ws || ws_bytes < need) {
         snprintf(g_detail, sizeof(g_detail), "workspace too small: need %zu bytes, got %zu", need, ws_bytes);
         return FLUE_ERR_WORKSPACE;
@@ -167,7 +179,11 @@ int energy_common(const flue_field* U, const PlaneSet& ps, int op, double* d_E, 
     if (!stage_timing_on()) {
         int nstream = 1;
         const int nslab = device_slabs(F.g, ps, &nstream);
-        if (nslab > 1 && ws_bytes >= energy_slabs_ws_bytes(F.g, F.prec, ps, d_force != nullptr, nslab, nstream))
+        // slabs with every intermediate; one pass with them; slabs in FP64 only
+        const bool all = ws_bytes >= energy_slabs_ws_bytes(F.g, F.prec, ps, d_force != nullptr, nslab, nstream);
+        const bool one = ws_bytes >= energy_ws_bytes(F.g, F.prec, ps, d_force != nullptr);
+        if (nslab > 1 && (all || (!one && ws_bytes >= energy_slabs_ws_min_bytes(F.g, F.prec, ps, d_force != nullptr,
+                                                                               nslab, nstream))))
             return cuda_status(
                 launch_energy_slabs(F, ps, d_E, d_force, form, ws, ws_bytes, nslab, nstream, (cudaStream_t)stream));
     }

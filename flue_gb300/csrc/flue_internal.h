@@ -84,7 +84,11 @@ struct PlaneSet {
     int np;
     int mu[6], nu[6];  // 0-based directions
 };
+// *_ws_bytes: the workspace an evaluation uses best; *_ws_min_bytes: the least
+// it accepts (complex128 fields then run in FP64 only, without the
+// fixed-point intermediates)
 size_t energy_ws_bytes(const Geom& g, int prec, const PlaneSet& ps, bool with_force);
+size_t energy_ws_min_bytes(const Geom& g, int prec, const PlaneSet& ps, bool with_force);
 cudaError_t launch_fmunu(const FieldRef& U, int kind, int mu, int nu, void* out, void* ws, size_t ws_bytes,
                          cudaStream_t st);
 cudaError_t launch_energy(const FieldRef& U, const PlaneSet& ps, double* out_E, void* force, int force_form, void* ws,
@@ -112,6 +116,7 @@ cudaError_t launch_energy_slab_out(const FieldRef& U, const PlaneSet& ps, int64_
 // energy_slabs_ws_bytes(...) bytes.  Results equal launch_energy's: the
 // gradient bitwise, the energy up to the order of the FP64 partial sums.
 size_t energy_slabs_ws_bytes(const Geom& g, int prec, const PlaneSet& ps, bool with_force, int nslab, int nstream);
+size_t energy_slabs_ws_min_bytes(const Geom& g, int prec, const PlaneSet& ps, bool with_force, int nslab, int nstream);
 cudaError_t launch_energy_slabs(const FieldRef& U, const PlaneSet& ps, double* out_E, void* force, int form, void* ws,
                                 size_t ws_bytes, int nslab, int nstream, cudaStream_t st);
 bool stage_timing_on();

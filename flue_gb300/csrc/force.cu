@@ -32,10 +32,12 @@
 //      Euclidean gradient N^+                              (k_linkcot)
 #include <stdlib.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "flue_internal.h"
 #include "loop5.cuh"
+#include "loop5_fix.cuh"
 
 namespace flue {
 
@@ -74,7 +76,7 @@ struct PatchArg {
     int tw, pm, pn, po;
 };
 
-__device__ __forceinline__ int64_t patch_site(const Geom& g, const PatchArg& pt, int pmu, int pnu, int64_t r) {
+__device__ __forceinline__ int64_t patch_site(const Geom& g, const PatchArg& pt, int pmu, int pnu, int64_t r, int tid) {
     int nm = 1, nn = 1;
     int64_t stm = 0, stn = 0, sto = 0;
     const int od = 6 - pmu - pnu;
@@ -91,7 +93,6 @@ __device__ __forceinline__ int64_t patch_site(const Geom& g, const PatchArg& pt,
     r /= nbm;
     const int bj = (int)(r % nbn);
     const int bo = (int)(r / nbn);
-    const int tid = threadIdx.x;
     const int tl = tid % pt.tw, pos = tid / pt.tw;
     const int im = pos % pt.pm, in = (pos / pt.pm) % pt.pn, io = pos / (pt.pm * pt.pn);
     return (int64_t)tc * pt.tw + tl + (int64_t)(bi * pt.pm + im) * stm + (int64_t)(bj * pt.pn + in) * stn +
@@ -137,6 +138,29 @@ __global__ void k_lines(L U, Geom g, Geom gs, int t0, PlaneArg pa, MatAoS<T> lin
     line_site<L, T>(U, g, gs, t0, pa, lines, s, (int)blockIdx.y);
 }
 
+// complex128 fields: the lines in fixed point (fix.cuh), counting the links
+// that are not unitary, or close to 1, in the gate.  32^3x64 B^2: 1.06 ms, HBM
+// (2.7 GB written) and the conversion of the links to limbs.
+__global__ void __launch_bounds__(128) k_lines_fix(FullLinks<double> U, Geom g, Geom gs, int t0, PlaneArg pa,
+                                                   MatFix lines, FixGate gt) {
+    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    u32 st = 0;
+    if (s < g.V) st = line_site_fix(U, g, gs, t0, pa, lines, s, (int)blockIdx.y);
+    gate_count(gt, st);
+}
+
+// The FP64 kernels behind a gate: every block leaves at once when the
+// fixed-point kernels have the field, else the (capped) grid walks the blocks
+// of the ungated grid.
+__device__ __forceinline__ bool gate_shut(const FixGate& gt) { return gt.p && gt.open(); }
+
+__global__ void __launch_bounds__(128) k_lines_gated(FullLinks<double> U, Geom g, Geom gs, int t0, PlaneArg pa,
+                                                     MatAoS<double> lines, FixGate gt) {
+    if (gate_shut(gt)) return;
+    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < g.V; s += (int64_t)gridDim.x * blockDim.x)
+        line_site<FullLinks<double>, double>(U, g, gs, t0, pa, lines, s, (int)blockIdx.y);
+}
+
 // ---------------------------------------------------------------------------
 // 2. forward: one thread per (site, plane)
 // ---------------------------------------------------------------------------
@@ -170,16 +194,31 @@ struct MinBlocks<float> {
     static constexpr int fwd = FLUE_FWD_MINB, cot = FLUE_COT_MINB;
 };
 constexpr int FWD_BS = FLUE_FWD_BS;
+// Sites a block of the fixed-point forward and line cotangents covers, three
+// threads a site: 384 threads and up to 168 registers, one block an SM.  Both
+// are bound by the integer multiply-add pipe (73% busy, waits on its results
+// next), so registers count for more than warps: B^2 force at 32^3x64 63.0 ms;
+// 64 sites with two blocks an SM 63.2, three (112 registers, spills) 67.6; 32
+// sites with four or five blocks 69.2, 69.9.
+#ifndef FLUE_FIX_BS
+#define FLUE_FIX_BS 128
+#endif
+constexpr int FIX_BS = FLUE_FIX_BS;
+
+// site j of the bs sites of block b of the forward's grid, plane p = b % np
+// (planes of the same site block run in adjacent blocks: L2 reuse)
+__device__ __forceinline__ int64_t fwd_site(const Geom& g, const PlaneArg& pa, const PatchArg& pt, unsigned b, int p,
+                                            int j, int bs) {
+    return pt.tw ? patch_site(g, pt, sel(pa.mu, p), sel(pa.nu, p), b / pa.np, j)
+                 : site_block(b / pa.np, g, bs) * bs + j;
+}
 
 template <typename T, typename I>
-__global__ void __launch_bounds__(FWD_BS, MinBlocks<T>::fwd)
-    k_fwd(Geom g, PlaneArg pa, int kind, PatchArg pt, MatAoS<T> lines, AHAoS<T> kout, RefOut<T> fout, double* part) {
-    __shared__ double sh[32];
-    // planes of the same site block run in adjacent blocks (L2 reuse)
-    const int p = blockIdx.x % pa.np;
-    const int pmu = sel(pa.mu, p), pnu = sel(pa.nu, p);
-    const int64_t s = pt.tw ? patch_site(g, pt, pmu, pnu, blockIdx.x / pa.np)
-                            : site_block(blockIdx.x / pa.np, g, blockDim.x) * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void fwd_block(unsigned b, const Geom& g, const PlaneArg& pa, int kind, const PatchArg& pt,
+                                          const MatAoS<T>& lines, const AHAoS<T>& kout, const RefOut<T>& fout,
+                                          double* part, double* sh) {
+    const int p = b % pa.np;
+    const int64_t s = fwd_site(g, pa, pt, b, p, threadIdx.x, blockDim.x);
     double e = 0.0;
     if (s < g.V) {
         int c[4];
@@ -189,6 +228,64 @@ __global__ void __launch_bounds__(FWD_BS, MinBlocks<T>::fwd)
         e = -(double)retr_mm<false, false>(f, f);
         if (kout.p) kout.store(s, p, f);
         if (fout.p) fout.store(s, 0, transp(f));
+    }
+    if (part) {
+        const double r = block_sum(e, sh);
+        if (threadIdx.x == 0) part[b] = r;
+    }
+}
+
+template <typename T, typename I>
+__global__ void __launch_bounds__(FWD_BS, MinBlocks<T>::fwd)
+    k_fwd(Geom g, PlaneArg pa, int kind, PatchArg pt, MatAoS<T> lines, AHAoS<T> kout, RefOut<T> fout, double* part) {
+    __shared__ double sh[32];
+    fwd_block<T, I>(blockIdx.x, g, pa, kind, pt, lines, kout, fout, part, sh);
+}
+
+template <typename I>
+__global__ void __launch_bounds__(FWD_BS)
+    k_fwd_gated(Geom g, PlaneArg pa, int kind, PatchArg pt, MatAoS<double> lines, AHAoS<double> kout,
+                RefOut<double> fout, double* part, unsigned nblocks, FixGate gt) {
+    __shared__ double sh[32];
+    if (gate_shut(gt)) return;
+    for (unsigned b = blockIdx.x; b < nblocks; b += gridDim.x)
+        fwd_block<double, I>(b, g, pa, kind, pt, lines, kout, fout, part, sh);
+}
+
+// Forward in fixed point: the sites and partial sums of the FP64 blocks, three
+// warps (columns) for every 32 sites.  32^3x64, three planes: FP64 pipe 81.1 ms,
+// fixed point with a thread a site 20.7 ms (240 registers, 8 warps an SM), with
+// a thread a column 19.0 ms.
+template <typename I>
+__global__ void __launch_bounds__(3 * FIX_BS)
+    k_fwd_fix(Geom g, PlaneArg pa, int kind, PatchArg pt, MatFix lines, AHFix kout, RefOut<double> fout, double* part,
+              u32* kmax, bool kslice, FixGate gt) {
+    __shared__ longlong2 sq[9][FIX_BS];
+    __shared__ double sh[32];
+    if (!gt.open()) return;
+    const int p = blockIdx.x % pa.np;
+    const int b = threadIdx.x / FIX_BS, j = threadIdx.x % FIX_BS;
+    const int64_t s = fwd_site(g, pa, pt, blockIdx.x, p, j, FIX_BS);
+    double e = 0.0;
+    int c[4];
+    if (s < g.V) {
+        site_coords(g, s, c);
+        const FxVS q = fwd_q_fix<I>(g, pa, kind, lines, s, c, p, b);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) sq[3 * a + b][j] = make_longlong2(q.r[a], q.i[a]);
+    }
+    __syncthreads();
+    if (b == 0 && s < g.V) {
+        i64 d[9];
+        fx_antiherm([&](int el) { return sq[el][j]; }, d);
+        double f[9];
+        fx_field_strength(d, kind == 1 ? FXQ5 : 1.0, f);
+        e = ah_norm2(f);
+        if (kout.p) {
+            kout.store(s, p, d);
+            kscale_max(kmax + (kslice ? c[0] : 0), e);
+        }
+        if (fout.p) fout.store(s, 0, transp(ah_expand(f)));
     }
     if (part) {
         const double r = block_sum(e, sh);
@@ -422,13 +519,13 @@ __device__ __forceinline__ void line_side(M3<T>& acc, M3<T>& X, T coef, const Ma
 }
 
 template <typename T, typename I>
-__global__ void __launch_bounds__(COT_BS, MinBlocks<T>::cot)
-    k_linecot(Geom g, PlaneArg pa, MatAoS<T> lines, AHAoS<T> kin, MatAoS<T> lam) {
+__device__ __forceinline__ void linecot_block(unsigned b, const Geom& g, const PlaneArg& pa, const MatAoS<T>& lines,
+                                              const AHAoS<T>& kin, const MatAoS<T>& lam) {
     // the 3 * nd (direction, length) tasks of one site block run in adjacent
     // blocks, so the neighbourhood they all read stays in L2
     const int ntask = 3 * pa.nd;
-    const int task = blockIdx.x % ntask;
-    const int64_t s64 = site_block(blockIdx.x / ntask, g, blockDim.x) * blockDim.x + threadIdx.x;
+    const int task = b % ntask;
+    const int64_t s64 = site_block(b / ntask, g, blockDim.x) * blockDim.x + threadIdx.x;
     if (s64 >= g.V) return;
     const I s = (I)s64;
     const int slot = task / 3;
@@ -474,6 +571,99 @@ __global__ void __launch_bounds__(COT_BS, MinBlocks<T>::cot)
     lam.store(s64, 3 * slot + len - 1, acc);
 }
 
+template <typename T, typename I>
+__global__ void __launch_bounds__(COT_BS, MinBlocks<T>::cot)
+    k_linecot(Geom g, PlaneArg pa, MatAoS<T> lines, AHAoS<T> kin, MatAoS<T> lam) {
+    linecot_block<T, I>(blockIdx.x, g, pa, lines, kin, lam);
+}
+
+template <typename I>
+__global__ void __launch_bounds__(COT_BS) k_linecot_gated(Geom g, PlaneArg pa, MatAoS<double> lines, AHAoS<double> kin,
+                                                          MatAoS<double> lam, unsigned nblocks, FixGate gt) {
+    if (gate_shut(gt)) return;
+    for (unsigned b = blockIdx.x; b < nblocks; b += gridDim.x) linecot_block<double, I>(b, g, pa, lines, kin, lam);
+}
+
+// line cotangents in fixed point: Lambda (180/512)^2 2^ks / 8, three warps
+// (columns) for every 32 sites.  X K(P) mixes the columns of X, which the three
+// warps exchange once a plane.  32^3x64: FP64 pipe 202 ms; a thread a site
+// 51.8 ms (its 255 registers spill), a thread a column 42.0 ms.
+template <typename I>
+__global__ void __launch_bounds__(3 * FIX_BS)
+    k_linecot_fix(Geom g, PlaneArg pa, MatFix lines, AHFix kin, MatFix lam, const u32* kmax, bool kslice, FixGate gt) {
+    __shared__ int4 sx[9][FIX_BS];
+    if (!gt.open()) return;
+    const int ntask = 3 * pa.nd;
+    const int task = blockIdx.x % ntask;
+    const int b = threadIdx.x / FIX_BS, jt = threadIdx.x % FIX_BS;
+    const int64_t s64 = site_block(blockIdx.x / ntask, g, FIX_BS) * FIX_BS + jt;
+    const bool live = s64 < g.V;
+    const I s = (I)(live ? s64 : 0);
+    const int slot = task / 3;
+    const int len = task % 3 + 1;
+    const int e = sel(pa.dir, slot);
+    int c[4];
+    site_coords(g, (int64_t)s, c);
+    int ce = 0, ne = 1;
+    int64_t ste = 1;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if (k == e) ce = c[k], ne = g.n[k], ste = g.st[k];
+    const I Q = s + (I)((int64_t)wrapd(ce, len, ne) * ste);
+    const int pB = 3 * slot + len - 1;
+    const int nw = len == 1 ? 3 : 2;
+    const int ks = kscale(kmax + (kslice ? c[0] : 0));
+    FxVS acc = vs_zero();
+#pragma unroll 1
+    for (int p = 0; p < pa.np; ++p) {
+        const int pmu = sel(pa.mu, p), pnu = sel(pa.nu, p);
+        if (pmu != e && pnu != e) continue;
+        const int f = pmu == e ? pnu : pmu;
+        int cf = 0, nf = 1;
+        int64_t stf = 1;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (k == f) cf = c[k], nf = g.n[k], stf = g.st[k];
+        const int kf = 3 * sel(pa.slot, f);
+        FxVS X = vs_zero();
+#pragma unroll 1
+        for (int j = 0; j < nw; ++j) {
+            const int w = c_lw_w[len - 1][j];
+            const int cw = pmu == e ? c_lw_n[len - 1][j] : -c_lw_n[len - 1][j];
+            const int pf = kf + w - 1;
+            line_side_fix<+1>(acc, X, cw, lines, kin, p, ks, s, Q, (I)((int64_t)wrapd(cf, w, nf) * stf), pf, pB, b);
+            line_side_fix<-1>(acc, X, cw, lines, kin, p, ks, s, Q, (I)((int64_t)wrapd(cf, -w, nf) * stf), pf, pB, b);
+        }
+        const FxV x = fx_of58(X);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) sx[3 * a + b][jt] = make_int4(x.r[a].h, x.r[a].l, x.i[a].h, x.i[a].l);
+        Fx kv[9];
+        kin.load(Q, p, ks, kv);
+        fx_add_kv(acc, kv, fx_prep<false>(x));
+        kin.load(s, p, ks, kv);
+        const FxVP kc = fx_prep<false>(ah_col(kv, b));
+        __syncthreads();
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            FxR m;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const int4 v = sx[3 * a + k][jt];
+                m.r[k] = {v.x, v.y};
+                m.i[k] = {v.z, v.w};
+            }
+            fx_row_sums<false>(m);
+            fx_rdot_add(acc, a, m, kc);
+        }
+        __syncthreads();
+    }
+    if (live) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+            lam.store_el(s64, 3 * slot + len - 1, 3 * a + b, fx_of61(acc.r[a]), fx_of61(acc.i[a]));
+    }
+}
+
 // ---------------------------------------------------------------------------
 // 4. link cotangents and gradient output: one thread per (site, direction),
 //    grid-strided so that a capped grid can write the gradient to host memory
@@ -481,7 +671,9 @@ __global__ void __launch_bounds__(COT_BS, MinBlocks<T>::cot)
 // ---------------------------------------------------------------------------
 template <typename T>
 __global__ void k_linkcot(Geom g, PlaneArg pa, MatAoS<T> lines, MatAoS<T> lam, T scale, int form, RefOut<T> out,
-                          bool skip_zero) {
+                          bool skip_zero, FixGate gt) {
+    if constexpr (sizeof(T) == 8)
+        if (gate_shut(gt)) return;
     const int d = blockIdx.y;
     const int slot = sel(pa.slot, d);
     if (slot < 0 && skip_zero) return;
@@ -520,6 +712,92 @@ __global__ void k_linkcot(Geom g, PlaneArg pa, MatAoS<T> lines, MatAoS<T> lam, T
     }
 }
 
+// link cotangents in fixed point: N (180/512)^2 2^ks / 8 from the stored
+// Lambda; the Lie form's U N takes N shifted up to |entry| < 1/2
+__global__ void __launch_bounds__(128) k_linkcot_fix(Geom g, PlaneArg pa, MatFix lines, MatFix lam, double scale,
+                                                     int form, RefOut<double> out, bool skip_zero,
+                                                     const u32* kmax, bool kslice, FixGate gt) {
+    if (!gt.open()) return;
+    const int d = blockIdx.y;
+    const int slot = sel(pa.slot, d);
+    if (slot < 0 && skip_zero) return;
+    for (int64_t z = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; z < g.V; z += (int64_t)gridDim.x * blockDim.x) {
+        if (slot < 0) {
+            out.store(z, d, m_zero<double>());
+            continue;
+        }
+        int c[4];
+        site_coords(g, z, c);
+        int cd = 0, nd = 1;
+        int64_t sd = 1;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (k == d) cd = c[k], nd = g.n[k], sd = g.st[k];
+        const int64_t zp = z + (int64_t)wrapd(cd, 1, nd) * sd, zm = z + (int64_t)wrapd(cd, -1, nd) * sd,
+                      zmm = z + (int64_t)wrapd(cd, -2, nd) * sd;
+        const int l1 = 3 * slot, l2 = 3 * slot + 1;
+        M3S n = s_zero();
+        {
+            const M3F up = lines.load(zp, l1);
+            fx_mac<false, false>(n, up, lam.load(z, 3 * slot + 1));
+            const M3F um = lines.load(zm, l1);
+            fx_mac<false, false>(n, fx_mm<false, false>(up, lam.load(zm, 3 * slot + 2)), um);
+            fx_mac<false, false>(n, lam.load(zm, 3 * slot + 1), um);
+        }
+        fx_mac<false, false>(n, lines.load(zp, l2), lam.load(z, 3 * slot + 2));
+        fx_mac<false, false>(n, lam.load(zmm, 3 * slot + 2), lines.load(zmm, l2));
+        {
+            const M3F l = lam.load(z, 3 * slot);
+#pragma unroll
+            for (int k = 0; k < 9; ++k) {
+                // h 2^-29 + l 2^-60 in units of 2^-58
+                n.r[k] += ((i64)l.r[k].h << 29) + (l.r[k].l >> 2);
+                n.i[k] += ((i64)l.i[k].h << 29) + (l.i[k].l >> 2);
+            }
+        }
+        // unit 2^-58 and the factors the fixed-point sums leave out
+        const double sc = ldexp(scale * (8.0 * FXQ5 * FXQ5) * 0x1p-58, -kscale(kmax + (kslice ? c[0] : 0)));
+        M3<double> o;
+        if (form == 0) {
+            u32 big = 0;
+#pragma unroll
+            for (int k = 0; k < 9; ++k)
+                big |= (u32)(n.r[k] >> 32) ^ (u32)(n.r[k] >> 63), big |= (u32)(n.i[k] >> 32) ^ (u32)(n.i[k] >> 63);
+            const int up = max(0, __clz((int)big) - 4);
+#pragma unroll
+            for (int k = 0; k < 9; ++k) n.r[k] <<= up, n.i[k] <<= up;
+            M3S un = s_zero();
+            fx_mac<false, false>(un, lines.load(z, l1), fx_of61(n));
+            // -1/2 TA: (M - M^+)/2 and a third of the trace off the diagonal
+            const double s1 = sc * -0.25 * ldexp(8.0, -up), s3 = sc * (-0.5 / 3.0) * ldexp(8.0, -up);
+            const i64 tr = un.i[0] + un.i[4] + un.i[8];
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+                o.r[4 * x] = 0.0;
+                o.i[4 * x] = (double)(3 * un.i[4 * x] - tr) * s3;
+#pragma unroll
+                for (int y = x + 1; y < 3; ++y) {
+                    const double cr = (double)(un.r[3 * x + y] - un.r[3 * y + x]) * s1;
+                    const double ci = (double)(un.i[3 * x + y] + un.i[3 * y + x]) * s1;
+                    o.r[3 * x + y] = cr;
+                    o.i[3 * x + y] = ci;
+                    o.r[3 * y + x] = -cr;
+                    o.i[3 * y + x] = ci;
+                }
+            }
+        } else {
+#pragma unroll
+            for (int x = 0; x < 3; ++x)
+#pragma unroll
+                for (int y = 0; y < 3; ++y) {
+                    o.r[3 * x + y] = (double)n.r[3 * y + x] * sc;
+                    o.i[3 * x + y] = (double)n.i[3 * y + x] * -sc;
+                }
+        }
+        out.store(z, d, o);
+    }
+}
+
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
@@ -544,26 +822,51 @@ static PlaneArg make_planes(const PlaneSet& ps) {
 static inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 struct EnergyWs {
-    size_t lines, kbuf, lam, part, total;
+    size_t lines, kbuf, lam, part, gate, gate_bytes, total;  // gate: its counts, then kscale's slices
+    bool fix;
 };
 
-static EnergyWs energy_layout(const Geom& g, int prec, const PlaneArg& pa, bool with_force) {
+// The scratch of one evaluation.  fix: complex128 fields with room for the
+// fixed-point intermediates (whole tiles of 32 sites) and the gate; they share
+// their place with the FP64 ones, since a field takes one of the two.
+static EnergyWs energy_layout(const Geom& g, int prec, const PlaneArg& pa, bool with_force, bool fix) {
     const bool d = prec == PREC_C128;  // FP64 intermediates
-    auto mat = [&](int64_t nk) { return d ? MatAoS<double>::bytes(g.V, nk) : MatAoS<float>::bytes(g.V, nk); };
-    auto ah = [&](int64_t nk) { return d ? AHAoS<double>::bytes(g.V, nk) : AHAoS<float>::bytes(g.V, nk); };
+    fix = fix && d;
+    auto mat = [&](int64_t nk) {
+        if (fix) return std::max(MatAoS<double>::bytes(g.V, nk), MatFix::bytes(g.V, nk));
+        return d ? MatAoS<double>::bytes(g.V, nk) : MatAoS<float>::bytes(g.V, nk);
+    };
+    auto ah = [&](int64_t nk) {
+        if (fix) return std::max(AHAoS<double>::bytes(g.V, nk), AHFix::bytes(g.V, nk));
+        return d ? AHAoS<double>::bytes(g.V, nk) : AHAoS<float>::bytes(g.V, nk);
+    };
     EnergyWs w;
-    const int nbx = (int)((g.V + FWD_BS - 1) / FWD_BS);
+    w.fix = fix;
+    const int fbs = fix ? FIX_BS : FWD_BS;
+    const int nbx = (int)((g.V + fbs - 1) / fbs);
     w.lines = 0;
     // daggered line copies only when the line cotangents run
     w.kbuf = align256(w.lines + mat(3 * pa.nd));
     w.lam = align256(w.kbuf + (with_force ? ah(pa.np) : 0));
     w.part = align256(w.lam + (with_force ? mat(3 * pa.nd) : 0));
-    w.total = align256(w.part + (size_t)pa.np * nbx * sizeof(double));
+    w.gate = align256(w.part + (size_t)pa.np * nbx * sizeof(double));
+    w.gate_bytes = fix ? (2 + (size_t)g.n[0]) * sizeof(u32) : 0;
+    w.total = align256(w.gate + w.gate_bytes);
     return w;
 }
 
+// the layout that fits ws_bytes: with the fixed-point intermediates, else
+// without (a workspace sized for the FP64 ones alone stays enough)
+static EnergyWs energy_layout_for(const Geom& g, int prec, const PlaneArg& pa, bool with_force, size_t ws_bytes) {
+    const EnergyWs w = energy_layout(g, prec, pa, with_force, true);
+    return ws_bytes >= w.total ? w : energy_layout(g, prec, pa, with_force, false);
+}
+
 size_t energy_ws_bytes(const Geom& g, int prec, const PlaneSet& ps, bool with_force) {
-    return energy_layout(g, prec, make_planes(ps), with_force).total;
+    return energy_layout(g, prec, make_planes(ps), with_force, true).total;
+}
+size_t energy_ws_min_bytes(const Geom& g, int prec, const PlaneSet& ps, bool with_force) {
+    return energy_layout(g, prec, make_planes(ps), with_force, false).total;
 }
 
 // Optional per-stage timing of the energy pipeline (CUDA events recorded on
@@ -607,6 +910,22 @@ static inline void stage_mark(int k, cudaStream_t st) {
     }
 }
 
+// The gate of one evaluation's workspace (p = NULL without the fixed-point
+// path): open when a quarter of its links is away from 1 and all are unitary.
+static FixGate energy_gate(const Geom& g, const PlaneArg& pa, char* ws, const EnergyWs& w) {
+    FixGate gt;
+    if (w.fix) {
+        gt.p = (u32*)(ws + w.gate);
+        gt.need = (u32)(((uint64_t)g.V * pa.nd + 3) / 4);
+    }
+    return gt;
+}
+// Grid of a gated FP64 kernel of n blocks: all of them when it always runs,
+// else at most 8 a SM, so that the blocks that leave at once cost little.
+static unsigned gated_grid(const EnergyWs& w, unsigned n) {
+    return w.fix ? std::min(n, 8u * (unsigned)device_sms()) : n;
+}
+
 // Part 1 of the pipeline: lines, forward (+ energy sum normalised by vnorm),
 // line cotangents when `with_force`.
 template <class L, typename T>
@@ -617,14 +936,41 @@ static cudaError_t energy_fwd_part(const L& U, const Geom& g, const Geom& gs, in
     AHAoS<T> kb{with_force ? reinterpret_cast<decltype(AHAoS<T>::p)>(ws + w.kbuf) : nullptr, g.V};
     MatAoS<T> lam{reinterpret_cast<decltype(MatAoS<T>::p)>(ws + w.lam), g.V};
     double* part = out_E ? (double*)(ws + w.part) : nullptr;
-    const unsigned nbx = (unsigned)((g.V + FWD_BS - 1) / FWD_BS);
+    const unsigned nbl = (unsigned)((g.V + 127) / 128);
+    const int fbs = w.fix ? FIX_BS : FWD_BS;  // sites a block of the forward covers
+    const unsigned nbx = (unsigned)((g.V + fbs - 1) / fbs);
+    const unsigned nbc = (unsigned)((g.V + COT_BS - 1) / COT_BS);
+    const PatchArg pt = FLUE_FWD_PATCH ? make_patch(g, pa, fbs) : PatchArg{};
+    const bool fits = MatAoS<T>::fits32(g.V, 3 * pa.nd), cfits = fits && AHAoS<T>::fits32(g.V, pa.np);
+    const bool ksl = pa.slot[0] < 0;  // no plane steps in time: one scale of K per time slice
+    cudaError_t e = cudaSuccess;
     stage_mark(0, st);
-    note_launch(), k_lines<L, T><<<dim3((unsigned)((g.V + 127) / 128), pa.nd), 128, 0, st>>>(U, g, gs, t0, pa, lines);
-    stage_mark(1, st);
-    const PatchArg pt = FLUE_FWD_PATCH ? make_patch(g, pa, FWD_BS) : PatchArg{};
-    const bool fits = MatAoS<T>::fits32(g.V, 3 * pa.nd);
-    bool tiled = false;
-    if constexpr (sizeof(T) == 4) {
+    if constexpr (sizeof(T) == 8) {
+        const FixGate gt = energy_gate(g, pa, ws, w);
+        const MatFix flines{(int4*)(ws + w.lines), g.V};
+        const AHFix fkb{with_force ? (longlong2*)(ws + w.kbuf) : nullptr, g.V};
+        const bool ffits = MatFix::fits32(g.V, 3 * pa.nd);
+        if (w.fix) {
+            if ((e = cudaMemsetAsync(gt.p, 0, w.gate_bytes, st)) != cudaSuccess) return e;
+            note_launch(), k_lines_fix<<<dim3(nbl, pa.nd), 128, 0, st>>>(U, g, gs, t0, pa, flines, gt);
+        }
+        note_launch(), k_lines_gated<<<dim3(gated_grid(w, nbl), pa.nd), 128, 0, st>>>(U, g, gs, t0, pa, lines, gt);
+        stage_mark(1, st);
+        if (w.fix) {
+            if (ffits)
+                note_launch(), k_fwd_fix<u32><<<nbx * pa.np, 3 * FIX_BS, 0, st>>>(g, pa, kind, pt, flines, fkb, fout, part, gt.p + 2, ksl, gt);
+            else
+                note_launch(), k_fwd_fix<int64_t><<<nbx * pa.np, 3 * FIX_BS, 0, st>>>(g, pa, kind, pt, flines, fkb, fout, part, gt.p + 2, ksl, gt);
+        }
+        const unsigned nf = nbx * pa.np, gf = gated_grid(w, nf);
+        if (fits)
+            note_launch(), k_fwd_gated<u32><<<gf, fbs, 0, st>>>(g, pa, kind, pt, lines, kb, fout, part, nf, gt);
+        else
+            note_launch(), k_fwd_gated<int64_t><<<gf, fbs, 0, st>>>(g, pa, kind, pt, lines, kb, fout, part, nf, gt);
+    } else {
+        note_launch(), k_lines<L, T><<<dim3(nbl, pa.nd), 128, 0, st>>>(U, g, gs, t0, pa, lines);
+        stage_mark(1, st);
+        bool tiled = false;
         if (fwd_tile_ok(g, pa, kind, fout.p != nullptr, fits)) {
             static_assert(FT_BS == FWD_BS, "the tile forward writes one partial per FWD_BS sites");
             // (the attribute is per function and per device; setting it again is harmless)
@@ -633,26 +979,42 @@ static cudaError_t energy_fwd_part(const L& U, const Geom& g, const Geom& gs, in
             note_launch(), k_fwd_tile<<<nbx * pa.np, FT_BS, FT_SMEM, st>>>(g, pa, lines, kb, part);
             tiled = true;
         }
+        if (!tiled) {
+            if (fits)
+                note_launch(), k_fwd<T, uint32_t><<<nbx * pa.np, FWD_BS, 0, st>>>(g, pa, kind, pt, lines, kb, fout, part);
+            else
+                note_launch(), k_fwd<T, int64_t><<<nbx * pa.np, FWD_BS, 0, st>>>(g, pa, kind, pt, lines, kb, fout, part);
+        }
     }
-    if (!tiled) {
-        if (fits)
-            note_launch(), k_fwd<T, uint32_t><<<nbx * pa.np, FWD_BS, 0, st>>>(g, pa, kind, pt, lines, kb, fout, part);
-        else
-            note_launch(), k_fwd<T, int64_t><<<nbx * pa.np, FWD_BS, 0, st>>>(g, pa, kind, pt, lines, kb, fout, part);
-    }
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (out_E) {
         e = launch_finish_sums(part, (int)(nbx * pa.np), 1, out_E, st, 1.0 / vnorm);
         if (e != cudaSuccess) return e;
     }
     stage_mark(2, st);
     if (!with_force) return cudaSuccess;
-    const unsigned nbc = (unsigned)((g.V + COT_BS - 1) / COT_BS);
-    if (MatAoS<T>::fits32(g.V, 3 * pa.nd) && AHAoS<T>::fits32(g.V, pa.np))
-        note_launch(), k_linecot<T, uint32_t><<<nbc * 3 * pa.nd, COT_BS, 0, st>>>(g, pa, lines, kb, lam);
-    else
-        note_launch(), k_linecot<T, int64_t><<<nbc * 3 * pa.nd, COT_BS, 0, st>>>(g, pa, lines, kb, lam);
+    if constexpr (sizeof(T) == 8) {
+        const FixGate gt = energy_gate(g, pa, ws, w);
+        const MatFix flines{(int4*)(ws + w.lines), g.V}, flam{(int4*)(ws + w.lam), g.V};
+        const AHFix fkb{(longlong2*)(ws + w.kbuf), g.V};
+        const unsigned nl = nbc * 3 * pa.nd, gl = gated_grid(w, nl);
+        const unsigned nlf = (unsigned)((g.V + FIX_BS - 1) / FIX_BS) * 3 * pa.nd;
+        if (w.fix) {
+            if (MatFix::fits32(g.V, 3 * pa.nd) && AHFix::fits32(g.V, pa.np))
+                note_launch(), k_linecot_fix<u32><<<nlf, 3 * FIX_BS, 0, st>>>(g, pa, flines, fkb, flam, gt.p + 2, ksl, gt);
+            else
+                note_launch(), k_linecot_fix<int64_t><<<nlf, 3 * FIX_BS, 0, st>>>(g, pa, flines, fkb, flam, gt.p + 2, ksl, gt);
+        }
+        if (cfits)
+            note_launch(), k_linecot_gated<u32><<<gl, COT_BS, 0, st>>>(g, pa, lines, kb, lam, nl, gt);
+        else
+            note_launch(), k_linecot_gated<int64_t><<<gl, COT_BS, 0, st>>>(g, pa, lines, kb, lam, nl, gt);
+    } else {
+        if (cfits)
+            note_launch(), k_linecot<T, uint32_t><<<nbc * 3 * pa.nd, COT_BS, 0, st>>>(g, pa, lines, kb, lam);
+        else
+            note_launch(), k_linecot<T, int64_t><<<nbc * 3 * pa.nd, COT_BS, 0, st>>>(g, pa, lines, kb, lam);
+    }
     stage_mark(3, st);
     return cudaGetLastError();
 }
@@ -667,7 +1029,18 @@ static cudaError_t energy_out_part(const Geom& g, const PlaneArg& pa, double vno
     const T scale = (T)(-1.0 / (2.0 * vnorm));
     unsigned nb = (unsigned)((g.V + 127) / 128);
     if (max_blocks && nb > max_blocks) nb = max_blocks;
-    note_launch(), k_linkcot<T><<<dim3(nb, 4), 128, 0, st>>>(g, pa, lines, lam, scale, form, fo, skip_zero);
+    FixGate gt;
+    unsigned nbg = nb;
+    if constexpr (sizeof(T) == 8) {
+        gt = energy_gate(g, pa, ws, w);
+        if (w.fix) {
+            const MatFix flines{(int4*)(ws + w.lines), g.V}, flam{(int4*)(ws + w.lam), g.V};
+            note_launch(), k_linkcot_fix<<<dim3(nb, 4), 128, 0, st>>>(g, pa, flines, flam, scale, form, fo, skip_zero,
+                                                                   gt.p + 2, pa.slot[0] < 0, gt);
+            nbg = gated_grid(w, nb);
+        }
+    }
+    note_launch(), k_linkcot<T><<<dim3(nbg, 4), 128, 0, st>>>(g, pa, lines, lam, scale, form, fo, skip_zero, gt);
     stage_mark(4, st);
     return cudaGetLastError();
 }
@@ -686,7 +1059,7 @@ static cudaError_t energy_impl(const L& U, const Geom& g, const PlaneArg& pa, in
 cudaError_t launch_energy(const FieldRef& U, const PlaneSet& ps, double* out_E, void* force, int force_form, void* ws,
                           size_t ws_bytes, cudaStream_t st) {
     const PlaneArg pa = make_planes(ps);
-    const EnergyWs w = energy_layout(U.g, U.prec, pa, force != nullptr);
+    const EnergyWs w = energy_layout_for(U.g, U.prec, pa, force != nullptr, ws_bytes);
     if (ws_bytes < w.total) return cudaErrorInvalidValue;
     FLUE_DISPATCH_LINKS(U, {
         RefOut<T> none{nullptr, U.g.V, 1};
@@ -707,7 +1080,7 @@ cudaError_t launch_energy_slab_fwd(const FieldRef& U, int t0, int nts, const Pla
     const Geom g = make_geom(nts, U.g.n[1], U.g.n[2], U.g.n[3]);
     if (vfull < g.V) return cudaErrorInvalidValue;
     const PlaneArg pa = make_planes(ps);
-    const EnergyWs w = energy_layout(g, U.prec, pa, with_force);
+    const EnergyWs w = energy_layout_for(g, U.prec, pa, with_force, ws_bytes);
     if (ws_bytes < w.total) return cudaErrorInvalidValue;
     FLUE_DISPATCH_LINKS(U, {
         RefOut<T> none{nullptr, g.V, 1};
@@ -722,7 +1095,7 @@ cudaError_t launch_energy_slab_out(const FieldRef& U, const PlaneSet& ps, int64_
                                    int out_dtype, bool skip_zero) {
     if (has_time_plane(ps) || vfull < U.g.V || t0 < 0 || t0 + U.g.n[0] > ntf) return cudaErrorInvalidValue;
     const PlaneArg pa = make_planes(ps);
-    const EnergyWs w = energy_layout(U.g, U.prec, pa, true);
+    const EnergyWs w = energy_layout_for(U.g, U.prec, pa, true, ws_bytes);
     if (ws_bytes < w.total) return cudaErrorInvalidValue;
     // the gradient array: time extent ntf, the slab's spatial extents (the
     // whole lattice's gradient, or a chunk of ntf time slices of it); vfull
@@ -784,11 +1157,11 @@ cudaError_t slab_streams(SlabStreams** out) {
 struct SlabWs {
     size_t slot, spart, total;
 };
-SlabWs slab_ws_layout(const Geom& g, int prec, const PlaneArg& pa, bool with_force, int nslab, int nstream) {
+SlabWs slab_ws_layout(const Geom& g, int prec, const PlaneArg& pa, bool with_force, int nslab, int nstream, bool fix) {
     const int nts = (g.n[0] + nslab - 1) / nslab;
     const Geom gs = make_geom(nts, g.n[1], g.n[2], g.n[3]);
     SlabWs w;
-    w.slot = energy_layout(gs, prec, pa, with_force).total;
+    w.slot = energy_layout(gs, prec, pa, with_force, fix).total;
     w.spart = (size_t)nstream * w.slot;
     w.total = align256(w.spart + (size_t)nslab * sizeof(double));
     return w;
@@ -797,8 +1170,11 @@ SlabWs slab_ws_layout(const Geom& g, int prec, const PlaneArg& pa, bool with_for
 
 bool stage_timing_on() { return g_stage_on; }
 
+size_t energy_slabs_ws_min_bytes(const Geom& g, int prec, const PlaneSet& ps, bool with_force, int nslab, int nstream) {
+    return slab_ws_layout(g, prec, make_planes(ps), with_force, nslab, nstream, false).total;
+}
 size_t energy_slabs_ws_bytes(const Geom& g, int prec, const PlaneSet& ps, bool with_force, int nslab, int nstream) {
-    return slab_ws_layout(g, prec, make_planes(ps), with_force, nslab, nstream).total;
+    return slab_ws_layout(g, prec, make_planes(ps), with_force, nslab, nstream, true).total;
 }
 
 cudaError_t launch_energy_slabs(const FieldRef& U, const PlaneSet& ps, double* out_E, void* force, int form, void* ws,
@@ -807,7 +1183,8 @@ cudaError_t launch_energy_slabs(const FieldRef& U, const PlaneSet& ps, double* o
         return cudaErrorInvalidValue;
     const PlaneArg pa = make_planes(ps);
     const bool with_force = force != nullptr;
-    const SlabWs w = slab_ws_layout(U.g, U.prec, pa, with_force, nslab, nstream);
+    SlabWs w = slab_ws_layout(U.g, U.prec, pa, with_force, nslab, nstream, true);
+    if (ws_bytes < w.total) w = slab_ws_layout(U.g, U.prec, pa, with_force, nslab, nstream, false);
     if (ws_bytes < w.total) return cudaErrorInvalidValue;
     const int nts = (U.g.n[0] + nslab - 1) / nslab;
     nslab = (U.g.n[0] + nts - 1) / nts;
@@ -850,7 +1227,7 @@ cudaError_t launch_fmunu(const FieldRef& U, int kind, int mu, int nu, void* out,
     ps.mu[0] = mu;
     ps.nu[0] = nu;
     const PlaneArg pa = make_planes(ps);
-    const EnergyWs w = energy_layout(U.g, U.prec, pa, false);
+    const EnergyWs w = energy_layout_for(U.g, U.prec, pa, false, ws_bytes);
     if (ws_bytes < w.total) return cudaErrorInvalidValue;
     FLUE_DISPATCH_LINKS(U, {
         using C2 = typename V2<T>::type;

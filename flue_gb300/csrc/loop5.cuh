@@ -81,20 +81,15 @@ __device__ __forceinline__ int wrapd(int c, int k, int n) {
 // Per-thread view of one plane (mu,nu) around the thread's site: every
 // coordinate the stencil needs is kept in scalars (no runtime-indexed
 // arrays, so nothing lands in local memory).
-template <typename T>
 struct Ctx {
-    MatAoS<T> lines;  // 3 per slot: L^1 (U expanded), L^2, L^3
     int64_t s;
     int cm, cn, nm, nn;  // coordinates and extents along mu, nu
     int64_t stm, stn;    // site strides along mu, nu
     int kmu, knu;        // first line plane of the mu / nu slot (3 * slot)
 };
 
-template <typename T>
-__device__ __forceinline__ Ctx<T> make_ctx(const MatAoS<T>& lines, const Geom& g, int64_t s, const int c[4], int mu,
-                                           int nu, int smu, int snu) {
-    Ctx<T> cx;
-    cx.lines = lines;
+__device__ __forceinline__ Ctx make_ctx(const Geom& g, int64_t s, const int c[4], int mu, int nu, int smu, int snu) {
+    Ctx cx;
     cx.s = s;
     // select without runtime indexing of c[] / g.n[] / g.st[]
 #pragma unroll
@@ -177,7 +172,7 @@ __device__ __forceinline__ void line_site(const L& U, const Geom& g, const Geom&
 // one.  The groups are the rows of c_lw_w / c_lw_c (a side of length len,
 // the other extent w).
 template <typename T, typename I>
-__device__ __forceinline__ M3<T> fwd_q5(const MatAoS<T>& lines, const Ctx<T>& cx) {
+__device__ __forceinline__ M3<T> fwd_q5(const MatAoS<T>& lines, const Ctx& cx) {
     const int s0 = (int)cx.s, stm = (int)cx.stm, stn = (int)cx.stn;
     auto ld = [&](int site, int k) { return ldm(lines, (I)site, k); };
     M3<T> q = m_zero<T>();
@@ -242,11 +237,11 @@ __device__ __forceinline__ M3<T> fwd_q(const Geom& g, const PlaneArg& pa, int ki
     // chains made its forward slower, 2.56 -> 2.72 ms at 32^3x64.
     if constexpr (sizeof(T) == 8) {
         if (kind == 1) {
-            const Ctx<T> cx5 = make_ctx(lines, g, s, c, pmu, pnu, sel(pa.slot, pmu), sel(pa.slot, pnu));
+            const Ctx cx5 = make_ctx(g, s, c, pmu, pnu, sel(pa.slot, pmu), sel(pa.slot, pnu));
             return fwd_q5<T, I>(lines, cx5);
         }
     }
-    const Ctx<T> cx = make_ctx(lines, g, s, c, pmu, pnu, sel(pa.slot, pmu), sel(pa.slot, pnu));
+    const Ctx cx = make_ctx(g, s, c, pmu, pnu, sel(pa.slot, pmu), sel(pa.slot, pnu));
     const Shape* shp = kind == 1 ? c_shapes5 : c_shapes1;
     const int nsh = kind == 1 ? 7 : 1;
     M3<T> q = m_zero<T>();

@@ -1,0 +1,119 @@
+"""Fixed-point products of complex128 fields (csrc/fix.cuh): B^2, its gradient
+and F_munu against the same entry points on a workspace that only holds the
+FP64 intermediates, at the edges of the 32-site tiles and 128-site blocks, and
+the fields that have to stay in FP64 (not unitary, not finite, close to 1).
+
+Bounds.  A fixed-point product is off by 2e-18 an entry and an FP64 one by
+2^-53 of its largest partial sum; the gradient passes about 40 products and the
+sums of 28 weighted leaves, so the two agree to a few times 40 2^-53 = 4e-15
+of the gradient's norm; B^2 sums V squares of either sign of error: 1e-14."""
+import ctypes
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+import oracle
+from flue_gb300 import _lib, generate
+from flue_gb300.field import as_field
+
+pytestmark = pytest.mark.gpu
+
+ALIGN = 256
+
+
+def _a(x):
+    return (x + ALIGN - 1) // ALIGN * ALIGN
+
+
+def _fp64_only_bytes(dims, nplanes, ndirs, force):
+    """What the FP64 intermediates take: lines, K, line cotangents, partials."""
+    v = int(np.prod(dims))
+    t = _a(3 * ndirs * v * 144)
+    t = _a(t + (nplanes * v * 80 if force else 0))
+    t = _a(t + (3 * ndirs * v * 144 if force else 0))
+    return _a(t + nplanes * ((v + 127) // 128) * 8)
+
+
+def _ptr(t):
+    return ctypes.c_void_p(t.data_ptr())
+
+
+def _energy(field, planes, form, nbytes):
+    nt, nx, ny, nz = field.dims
+    p = np.ascontiguousarray(np.asarray(planes, dtype=np.int32).reshape(-1))
+    ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+    e = torch.empty(1, dtype=torch.float64, device="cuda")
+    g = torch.empty((3, 3, 4, nz, ny, nx, nt), dtype=torch.complex128, device="cuda")
+    d = field.descriptor()
+    _lib.call("flue_loop5_energy_force", ctypes.byref(d), p.ctypes.data_as(ctypes.c_void_p), len(planes), _ptr(e),
+              _ptr(g), form, _ptr(ws), nbytes, ctypes.c_void_p(0))
+    torch.cuda.synchronize()
+    return e.item(), g.cpu().numpy()
+
+
+def _both(field, planes, form):
+    dirs = len({d for p in planes for d in p})
+    small = _fp64_only_bytes(field.dims, len(planes), dirs, True)
+    full = max(_lib.load().flue_workspace_bytes(op, *field.dims, _lib.C128)
+               for op in (_lib.OP_MAGNETIC_FORCE, _lib.OP_ENERGY_FORCE))
+    assert full > small
+    return _energy(field, planes, form, full), _energy(field, planes, form, small)
+
+
+B2 = ((3, 2), (2, 4), (4, 3))
+ALL = ((1, 2), (1, 3), (1, 4), (2, 3), (2, 4), (3, 4))
+
+
+# 31, 32, 33, 127, 128, 129 sites among the volumes; extents down to 1 and 2
+@pytest.mark.parametrize("dims", [(31, 1, 1, 1), (4, 2, 2, 2), (3, 11, 1, 1), (127, 1, 1, 1), (8, 4, 2, 2), (43, 3, 1, 1),
+                                  (5, 3, 4, 7), (16, 8, 8, 8)])
+@pytest.mark.parametrize("planes", [B2, ALL, ((1, 4),)])
+@pytest.mark.parametrize("eps", [0.0, 0.1, 0.4])
+def test_fixed_point_against_fp64(dims, planes, eps):
+    u = generate.haar_field(dims, 5) if eps == 0.0 else generate.random_field(dims, eps, 5)
+    f = as_field(u)
+    for form in (_lib.FORCE_LIE, _lib.FORCE_EUCLID):
+        (e1, g1), (e0, g0) = _both(f, planes, form)
+        assert abs(e1 - e0) <= 1e-14 * abs(e0) + 1e-28
+        # (extents of 1 and 2 make some gradients vanish up to rounding)
+        scale = max(np.linalg.norm(g0), np.sqrt(g0.size) * 1e-3 / np.prod(dims))
+        assert np.linalg.norm(g1 - g0) <= 8e-15 * scale
+
+
+@pytest.mark.parametrize("change", ["scaled", "nan", "inf", "not_orthogonal", "cold", "near_cold", "huge"])
+def test_fields_that_stay_in_fp64(change):
+    dims = (7, 5, 4, 3)
+    u = np.array(generate.random_field(dims, 0.3, 9))
+    if change == "scaled":
+        u[3, 2, 1, 0, 2] *= 1.01
+    elif change in ("nan", "inf"):
+        u[3, 2, 1, 0, 2, 1, 1] = np.nan if change == "nan" else np.inf
+    elif change == "not_orthogonal":
+        u[0, 0, 0, 0, 1, 1] = u[0, 0, 0, 0, 1, 0]
+    elif change == "huge":
+        u[3, 2, 1, 0, 3, 0, 0] = 1e300
+    elif change == "cold":
+        u = np.array(generate.cold_field(dims))
+    else:
+        u = np.array(generate.random_field(dims, 1e-3, 9))
+    (e1, g1), (e0, g0) = _both(as_field(np.asfortranarray(u)), B2, _lib.FORCE_LIE)
+    assert np.array_equal(e1, e0, equal_nan=True) and np.array_equal(g1, g0, equal_nan=True)
+
+
+def test_rough_fields_take_fixed_point():
+    f = as_field(generate.random_field((8, 6, 4, 4), 0.3, 2))
+    (_, g1), (_, g0) = _both(f, B2, _lib.FORCE_LIE)
+    assert not np.array_equal(g1, g0)
+
+
+def test_gauge_fixed_time_links_take_fixed_point():
+    """A quarter of the links at 1 (temporal gauge) does not shut the gate."""
+    u = np.array(generate.random_field((8, 6, 4, 4), 0.3, 2))
+    u[..., 0, :, :] = np.eye(3)
+    f = as_field(np.asfortranarray(u))
+    (e1, g1), (e0, g0) = _both(f, ALL, _lib.FORCE_LIE)
+    assert not np.array_equal(g1, g0)
+    assert np.linalg.norm(g1 - g0) <= 8e-15 * np.linalg.norm(g0)
+    assert abs(e1 - oracle.loop5_energy(u, ALL)) <= 1e-12 * abs(e0)

@@ -110,7 +110,7 @@ size_t ws_bytes_for(int op, const Geom& g, int prec) {
         case FLUE_OP_MEANLINK:
             return a256((size_t)meanlink_slots(g) * 4 * 8);
         case FLUE_OP_WFLOW:
-            return wflow_ws_bytes(g);
+            return wflow_ws_bytes(g, prec);
         case FLUE_OP_GLUON_PROP:
             return gluon_prop_ws_bytes(g, prec);
         default:
@@ -127,6 +127,7 @@ size_t ws_min_bytes_for(int op, const Geom& g, int prec) {
         ps.nu[0] = 1;
         return energy_ws_min_bytes(g, prec, ps, false);
     }
+    if (op == FLUE_OP_WFLOW) return wflow_ws_min_bytes(g);
     return ws_bytes_for(op, g, prec);
 }
 
@@ -461,7 +462,7 @@ int flue_wflow_step(const flue_field* U, double eps, void* ws, size_t ws_bytes, 
     if (F.prec == FLUE_R12) return fail(FLUE_ERR_DTYPE, "Wilson flow needs a C128 or C64 field");
     if (!(eps > 0.0) || !isfinite(eps)) return fail(FLUE_ERR_ARG, "eps must be positive");
     if ((rc = check_ws(FLUE_OP_WFLOW, F, ws_bytes, ws))) return rc;
-    return cuda_status(launch_wflow_step((void*)F.links, F.g, F.prec, eps, ws, (cudaStream_t)stream));
+    return cuda_status(launch_wflow_step((void*)F.links, F.g, F.prec, eps, ws, ws_bytes, (cudaStream_t)stream));
 }
 
 }  // extern "C"

@@ -72,6 +72,9 @@ __device__ __forceinline__ Fx fx_of61(i64 s) {
     return r;
 }
 
+// the value as one integer of unit 2^-60
+__device__ __forceinline__ i64 fx_int60(const Fx& a) { return ((i64)a.h << 31) + a.l; }
+
 // double to Fx, |x| < 2: the 53-bit significand shifted to unit 2^-60
 // (truncated below it), without an FP64 instruction
 __device__ __forceinline__ Fx fx_of(double x) {
@@ -327,6 +330,9 @@ struct FixGate {
         return *(volatile const u32*)p == 0 && ((volatile const u32*)p)[1] >= need;
     }
 };
+// whether the FP64 kernels behind a gate have nothing to do (without a gate
+// they always run)
+__device__ __forceinline__ bool gate_shut(const FixGate& gt) { return gt.p && gt.open(); }
 // A quarter of the links has to be further than 1/16 from 1 (Frobenius norm):
 // closer to 1 the FP64 products keep more bits of the small off-diagonal and
 // imaginary parts than fixed point does.  (A quarter: a gauge fixed along one
@@ -544,6 +550,24 @@ __device__ __forceinline__ FxV ah_col(const Fx v[9], int b) {
 __device__ __forceinline__ void fx_add_kv(FxVS& S, const Fx k[9], const FxVP& v) {
 #pragma unroll
     for (int a = 0; a < 3; ++a) fx_rdot_add(S, a, ah_row(k, a), v);
+}
+
+// the anti-Hermitian q - q^+ as 9 integers of q's unit, in the order of AHFix;
+// q(e) is entry e = 3 a + b
+template <class Q>
+__device__ __forceinline__ void fx_antiherm(Q q, i64 d[9]) {
+    d[0] = 2 * q(0).y;
+    d[1] = 2 * q(4).y;
+    d[2] = 2 * q(8).y;
+    longlong2 u = q(1), l = q(3);
+    d[3] = u.x - l.x;
+    d[4] = u.y + l.y;
+    u = q(2), l = q(6);
+    d[5] = u.x - l.x;
+    d[6] = u.y + l.y;
+    u = q(5), l = q(7);
+    d[7] = u.x - l.x;
+    d[8] = u.y + l.y;
 }
 
 }  // namespace flue

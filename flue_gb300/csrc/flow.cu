@@ -16,17 +16,39 @@
 // small D apart from I holds its relative precision in FP32, so the update
 // adds one rounding of W per stage, as an FP64 update rounded to FP32 would.
 // FP32 fields are reunitarised (FixSU3Matrix) after every stage.
+#include <math.h>
+
+#include <algorithm>
+
 #include "flue_internal.h"
 
 namespace flue {
 
-size_t wflow_ws_bytes(const Geom& g) {
+size_t wflow_ws_min_bytes(const Geom& g) {
     // force (4 x 9 complex doubles per site), B (4 x 9 reals per site),
     // plaquette partials
     const size_t f = (size_t)36 * g.V * 16;
     const size_t b = (size_t)36 * g.V * 8;
     const size_t p = (size_t)plaqforce_blocks(g) * 4 * 8;
     return ((f + 255) & ~(size_t)255) + ((b + 255) & ~(size_t)255) + ((p + 255) & ~(size_t)255);
+}
+
+// the fixed-point step's scratch: two link fields, X of the last stage, the
+// gate (the FP64 step's buffers, used when the gate is shut, lie over the
+// fields)
+struct FlowFixWs {
+    size_t w1, x, gate, total;
+};
+static FlowFixWs flow_fix_layout(const Geom& g) {
+    FlowFixWs w;
+    w.w1 = MatFix::bytes(g.V, 4);
+    w.x = w.w1 + MatFix::bytes(g.V, 4);
+    w.gate = std::max(w.x + AHFix::bytes(g.V, 4), wflow_ws_min_bytes(g));
+    w.total = w.gate + 256;
+    return w;
+}
+size_t wflow_ws_bytes(const Geom& g, int prec) {
+    return prec == PREC_C128 ? flow_fix_layout(g).total : wflow_ws_min_bytes(g);
 }
 
 template <typename T>
@@ -249,10 +271,8 @@ __device__ __forceinline__ void reunitarise(M3<W>& w) {
 }
 
 template <typename T>
-__global__ void k_wflow_update(void* links, Geom g, const void* force, AHPlanes<T> bbuf, T eps, int stage,
-                               int reun) {
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= 4 * g.V) return;
+__device__ __forceinline__ void wflow_update(int64_t idx, void* links, const Geom& g, const void* force,
+                                             const AHPlanes<T>& bbuf, T eps, int stage, int reun) {
     const int64_t s = idx % g.V;
     const int mu = (int)(idx / g.V);
     // Z = eps * 2 G, G in the field's compute type, same layout as the field
@@ -290,7 +310,206 @@ __global__ void k_wflow_update(void* links, Geom g, const void* force, AHPlanes<
         }
 }
 
-cudaError_t launch_wflow_step(void* links, const Geom& g, int prec, double eps, void* ws, cudaStream_t st) {
+template <typename T>
+__global__ void k_wflow_update(void* links, Geom g, const void* force, AHPlanes<T> bbuf, T eps, int stage, int reun,
+                               FixGate gt) {
+    int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if constexpr (sizeof(T) == 8) {  // capped grid when gated
+        if (gate_shut(gt)) return;
+        for (; idx < 4 * g.V; idx += (int64_t)gridDim.x * blockDim.x)
+            wflow_update<T>(idx, links, g, force, bbuf, eps, stage, reun);
+    } else if (idx < 4 * g.V) {
+        wflow_update<T>(idx, links, g, force, bbuf, eps, stage, reun);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The step of a complex128 field in fixed point (fix.cuh): the links are
+// converted once (k_flow_links), each stage computes the force of a link and
+// moves it in one kernel from one fixed-point field to the other, and the last
+// stage writes the complex128 links.  A thread carries one column of a link
+// (three warps for 32 sites), as the 5-loop kernels do.  A stage is 13 matrix
+// products and the Taylor terms of exp(X) a link, bound by the integer
+// multiply-add pipe; 24^3x48: 13.5 ms as FP64 force and update, 2.4 ms so.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(128) k_flow_links(FullLinks<double> U, Geom g, MatFix w, FixGate gt) {
+    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    u32 st = 0;
+    if (s < g.V) {
+        const M3<double> u = U.load(s, (int)blockIdx.y);
+        st = link_state(u);
+        w.store(s, (int)blockIdx.y, fx_of(u));
+    }
+    gate_count(gt, st);
+}
+
+// a value of unit 2^-60 as limbs
+__host__ __device__ constexpr Fx fx_const60(i64 x) {
+    return {(int)((x + ((i64)1 << 30)) >> 31), (int)(x - ((x + ((i64)1 << 30)) >> 31) * ((i64)1 << 31))};
+}
+static Fx fx_const(double x) { return fx_const60((i64)llrint(ldexp(x, 60))); }
+// 1/k!
+constexpr int FLOW_TERMS = 20;
+struct FlowFact {
+    Fx f[FLOW_TERMS + 1];
+};
+constexpr FlowFact flow_fact() {
+    FlowFact t{};
+    i64 fact = 1;  // 20! < 2^62
+    for (int k = 0; k <= FLOW_TERMS; ++k) {
+        if (k) fact *= k;
+        t.f[k] = fx_const60((((i64)1 << 60) + fact / 2) / fact);
+    }
+    return t;
+}
+static __constant__ FlowFact c_flow_fact = flow_fact();
+
+// X of a stage: the off-diagonal and diagonal factor of the projected U N and
+// the factor of the last stage's X
+struct FlowStage {
+    Fx off, diag, last;
+};
+constexpr int FF_BS = 128;  // sites a block
+
+template <int STAGE, typename I>
+__global__ void __launch_bounds__(3 * FF_BS)
+    k_flow_stage(Geom g, MatFix w, MatFix wout, AHFix xb, FlowStage sc, double2* links, FixGate gt) {
+    __shared__ longlong2 sq[9][FF_BS];
+    if (!gt.open()) return;
+    const int mu = blockIdx.x & 3;  // the directions of a site block in adjacent blocks (L2 reuse)
+    const int b = threadIdx.x / FF_BS, j = threadIdx.x % FF_BS;
+    const int64_t s64 = (int64_t)(blockIdx.x >> 2) * FF_BS + j;
+    const bool live = s64 < g.V;
+    const I s = (I)(live ? s64 : 0);
+    int c[4];
+    site_coords(g, (int64_t)s, c);
+    I fw[4], bw[4];  // steps of +-1
+#pragma unroll
+    for (int d = 0; d < 4; ++d) {
+        fw[d] = (I)(c[d] + 1 == g.n[d] ? -(int64_t)(g.n[d] - 1) * g.st[d] : g.st[d]);
+        bw[d] = (I)(c[d] == 0 ? (int64_t)(g.n[d] - 1) * g.st[d] : -g.st[d]);
+    }
+    I fm = fw[0];
+#pragma unroll
+    for (int d = 1; d < 4; ++d)
+        if (d == mu) fm = fw[d];
+    // column b of N, the sum of the six staples: |N| <= 6
+    FxVS n = vs_zero();
+#pragma unroll 1
+    for (int k = 1; k < 4; ++k) {
+        const int nu = (mu + k) & 3;
+        I fn = fw[0], bn = bw[0];
+#pragma unroll
+        for (int d = 1; d < 4; ++d)
+            if (d == nu) fn = fw[d], bn = bw[d];
+        FxV v = w.mul<true>((I)(s + fn), mu, w.col<true>(s, nu, b));
+        w.mac<false>(n, (I)(s + fm), nu, v);
+        v = w.mul<true>((I)(s + bn), mu, w.col<false>((I)(s + bn), nu, b));
+        w.mac<true>(n, (I)(s + fm + bn), nu, v);
+    }
+    {  // U N / 8
+        FxV v;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) v.r[a] = fx_of61(n.r[a]), v.i[a] = fx_of61(n.i[a]);
+        FxVS un = vs_zero();
+        w.mac<false>(un, s, mu, v);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) sq[3 * a + b][j] = make_longlong2(un.r[a], un.i[a]);
+    }
+    __syncthreads();
+    // X = sc . (U N - (U N)^+ without its trace) + sc.last X_last
+    Fx x[9];
+    {
+        i64 d[9];
+        fx_antiherm([&](int el) { return sq[el][j]; }, d);
+        // (diagonal entries of fx_antiherm are 2 Im: 3 Im - trace from them)
+        const i64 tr = (d[0] + d[1] + d[2]) >> 1;
+        Fx last[9];
+        if (STAGE > 0) xb.load(s, mu, 0, last);
+#pragma unroll
+        for (int e = 0; e < 9; ++e) {
+            const i64 de = e < 3 ? d[e] + (d[e] >> 1) - tr : d[e];
+            FxAcc t = {FX_HI0, FX_CR0};
+            fx_mad(t, fx_of61(de), e < 3 ? sc.diag : sc.off);
+            if (STAGE > 0) fx_mad(t, last[e], sc.last);
+            x[e] = fx_limbs(t);
+        }
+        if (STAGE < 2 && live && b == 0) {
+#pragma unroll
+            for (int e = 0; e < 9; ++e) d[e] = ((i64)x[e].h << 32) + 2 * (i64)x[e].l;
+            xb.store(s64, mu, d);
+        }
+    }
+    // exp(X) U by Taylor on the column, X halved until |X|_F <= 1/2
+    float nrm = 0.f;
+#pragma unroll
+    for (int e = 0; e < 9; ++e) {
+        const float t = (float)x[e].h * 0x1p-29f;
+        nrm = fmaf(e < 3 ? t : 2.f * t, t, nrm);
+    }
+    nrm = sqrtf(nrm) * 1.0001f;
+    int reps = 1;
+    while (nrm > 0.5f && reps < 64) {
+        nrm *= 0.5f;
+        reps *= 2;
+#pragma unroll
+        for (int e = 0; e < 9; ++e) x[e] = fx_of61((((i64)x[e].h << 32) + 2 * (i64)x[e].l) >> 1);
+    }
+    FxV u = w.col<false>(s, mu, b);
+#pragma unroll 1
+    for (int rep = 0; rep < reps; ++rep) {
+        FxAcc sr[3], si[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) sr[a] = si[a] = {FX_HI0, FX_CR0};
+        FxV t = u;
+        float bnd = 1.f;
+#pragma unroll 1
+        for (int k = 1; k <= FLOW_TERMS; ++k) {
+            bnd *= nrm / (float)k;
+            if (!(bnd > 0x1p-62f)) break;
+            const FxVP tp = fx_prep<false>(t);
+#pragma unroll
+            for (int a = 0; a < 3; ++a) fx_rdot_limbs(t.r[a], t.i[a], ah_row(x, a), tp);
+#pragma unroll
+            for (int a = 0; a < 3; ++a) fx_mad(sr[a], t.r[a], c_flow_fact.f[k]), fx_mad(si[a], t.i[a], c_flow_fact.f[k]);
+        }
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            u.r[a] = fx_const60(fx_int60(u.r[a]) + fx_int60(fx_limbs(sr[a])));
+            u.i[a] = fx_const60(fx_int60(u.i[a]) + fx_int60(fx_limbs(si[a])));
+        }
+    }
+    if (!live) return;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        if (STAGE < 2) {
+            wout.store_el(s64, mu, 3 * a + b, u.r[a], u.i[a]);
+        } else if (FLUE_INB(s64 < g.V)) {
+            links[s64 + g.V * (mu + 4 * (a + 3 * b))] =
+                make_double2((double)fx_int60(u.r[a]) * 0x1p-60, (double)fx_int60(u.i[a]) * 0x1p-60);
+        }
+    }
+}
+
+template <typename I>
+static void flow_fix_stages(void* links, const Geom& g, double eps, char* ws, const FlowFixWs& w, const FixGate& gt,
+                            cudaStream_t st) {
+    const MatFix w0{(int4*)ws, g.V}, w1{(int4*)(ws + w.w1), g.V};
+    const AHFix xb{(longlong2*)(ws + w.x), g.V};
+    const unsigned nb = (unsigned)((g.V + FF_BS - 1) / FF_BS) * 4;
+    // Z = -eps TA(U N): the kernel holds (U N - (U N)^+)/64 off the diagonal and
+    // (3 Im - trace)/64 on it.  The kept X of stage 0 is Z0/4, so stage 1 takes
+    // 8/9 Z1 - 17/36 (4 X) and stage 2 takes 3/4 Z2 - X.
+    const double f[3] = {0.25, 8.0 / 9.0, 0.75}, last[3] = {0.0, -17.0 / 9.0, -1.0};
+    FlowStage sc[3];
+    for (int k = 0; k < 3; ++k) sc[k] = {fx_const(-32.0 * eps * f[k]), fx_const(-64.0 / 3.0 * eps * f[k]), fx_const(last[k])};
+    note_launch(), k_flow_stage<0, I><<<nb, 3 * FF_BS, 0, st>>>(g, w0, w1, xb, sc[0], nullptr, gt);
+    note_launch(), k_flow_stage<1, I><<<nb, 3 * FF_BS, 0, st>>>(g, w1, w0, xb, sc[1], nullptr, gt);
+    note_launch(), k_flow_stage<2, I><<<nb, 3 * FF_BS, 0, st>>>(g, w0, w1, xb, sc[2], (double2*)links, gt);
+}
+
+cudaError_t launch_wflow_step(void* links, const Geom& g, int prec, double eps, void* ws, size_t ws_bytes,
+                              cudaStream_t st) {
     char* w = (char*)ws;
     const size_t f = (((size_t)36 * g.V * 16) + 255) & ~(size_t)255;
     const size_t b = (((size_t)36 * g.V * 8) + 255) & ~(size_t)255;
@@ -301,13 +520,33 @@ cudaError_t launch_wflow_step(void* links, const Geom& g, int prec, double eps, 
     double* part = (double*)(w + f + b);
     FieldRef U{links, g, prec};
     const unsigned nb = (unsigned)((4 * g.V + 127) / 128);
-    for (int stage = 0; stage < 3; ++stage) {
-        cudaError_t e = launch_plaquette_force(U, part, nullptr, force, 0, st);
+    // Fixed point for complex128 fields with its workspace; its factors leave
+    // their range (|32 eps| < 4) at eps = 1/8, where a step is far too long anyway.
+    const FlowFixWs fw = flow_fix_layout(g);
+    FixGate gt;
+    if (prec == PREC_C128 && ws_bytes >= fw.total && eps < 0.12) {
+        gt.p = (u32*)(w + fw.gate);
+        gt.need = (u32)g.V;  // a quarter of the links
+        cudaError_t e = cudaMemsetAsync(gt.p, 0, 2 * sizeof(u32), st);
         if (e != cudaSuccess) return e;
-        if (prec == PREC_C128)
-            note_launch(), k_wflow_update<double><<<nb, 128, 0, st>>>(links, g, force, bb, eps, stage, 0);
+        const MatFix w0{(int4*)w, g.V};
+        note_launch(), k_flow_links<<<dim3((unsigned)((g.V + 127) / 128), 4), 128, 0, st>>>(
+            FullLinks<double>{(const double2*)links, g.V}, g, w0, gt);
+        if (MatFix::fits32(g.V, 4))
+            flow_fix_stages<u32>(links, g, eps, w, fw, gt, st);
         else
-            note_launch(), k_wflow_update<float><<<nb, 128, 0, st>>>(links, g, force, bbf, (float)eps, stage, 1);
+            flow_fix_stages<int64_t>(links, g, eps, w, fw, gt, st);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    for (int stage = 0; stage < 3; ++stage) {
+        cudaError_t e = gt.p ? launch_plaquette_force_gated(U, force, gt, st)
+                             : launch_plaquette_force(U, part, nullptr, force, 0, st);
+        if (e != cudaSuccess) return e;
+        const unsigned nbg = gt.p ? std::min(nb, 8u * (unsigned)device_sms()) : nb;
+        if (prec == PREC_C128)
+            note_launch(), k_wflow_update<double><<<nbg, 128, 0, st>>>(links, g, force, bb, eps, stage, 0, gt);
+        else
+            note_launch(), k_wflow_update<float><<<nb, 128, 0, st>>>(links, g, force, bbf, (float)eps, stage, 1, gt);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }

@@ -6,6 +6,7 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include "fix.cuh"
 #include "flue_common.cuh"
 
 struct flue_field;
@@ -123,6 +124,9 @@ bool stage_timing_on();
 int plaqforce_blocks(const Geom& g);
 cudaError_t launch_plaquette_force(const FieldRef& U, double* part, double* out_S, void* force, int force_form,
                                    cudaStream_t st);
+// Lie-form force of a complex128 field, run only where the gate is shut for
+// fixed point
+cudaError_t launch_plaquette_force_gated(const FieldRef& U, void* force, const FixGate& gt, cudaStream_t st);
 
 // out-of-bounds counters of the bounds-checked build, one per translation
 // unit (read and cleared; 0 in the normal build)
@@ -156,8 +160,10 @@ cudaError_t stage_timing_enable(int on);
 cudaError_t stage_times(double* ms, int maxn, int* n);
 
 // Wilson flow (flow.cu)
-size_t wflow_ws_bytes(const Geom& g);
-cudaError_t launch_wflow_step(void* links, const Geom& g, int prec, double eps, void* ws, cudaStream_t st);
+size_t wflow_ws_bytes(const Geom& g, int prec);
+size_t wflow_ws_min_bytes(const Geom& g);
+cudaError_t launch_wflow_step(void* links, const Geom& g, int prec, double eps, void* ws, size_t ws_bytes,
+                              cudaStream_t st);
 
 // gauge transformation and gluon propagator (propagator.cu)
 cudaError_t launch_gauge_transform(const FieldRef& U, const void* G, int g_dtype, cudaStream_t st);

@@ -150,10 +150,8 @@ __global__ void __launch_bounds__(128) k_lines_fix(FullLinks<double> U, Geom g, 
 }
 
 // The FP64 kernels behind a gate: every block leaves at once when the
-// fixed-point kernels have the field, else the (capped) grid walks the blocks
-// of the ungated grid.
-__device__ __forceinline__ bool gate_shut(const FixGate& gt) { return gt.p && gt.open(); }
-
+// fixed-point kernels have the field (gate_shut), else the (capped) grid walks
+// the blocks of the ungated grid.
 __global__ void __launch_bounds__(128) k_lines_gated(FullLinks<double> U, Geom g, Geom gs, int t0, PlaneArg pa,
                                                      MatAoS<double> lines, FixGate gt) {
     if (gate_shut(gt)) return;
@@ -1288,16 +1286,16 @@ struct PfMinBlocks<R12Links, float> {
     static constexpr int v = 4;
 };
 
+// block b of nb (the grid's x) of direction d
 template <class L, typename T>
-__global__ void __launch_bounds__(PF_BS, PfMinBlocks<L, T>::v)
-    k_plaqforce(L U, Geom g, int form, RefOut<T> out, double* part) {
-    __shared__ double sh[32];
-    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void plaqforce_block(unsigned b, unsigned nb, int d, const L& U, const Geom& g, int form,
+                                                const RefOut<T>& out, double* part, double* sh) {
+    const int64_t s = (int64_t)b * blockDim.x + threadIdx.x;
     double acc = 0.0;
     if (s < g.V) {
         int c[4];
         site_coords(g, s, c);
-        switch (blockIdx.y) {
+        switch (d) {
             case 0: acc = plaqforce_dir<0>(U, g, s, c, form, out); break;
             case 1: acc = plaqforce_dir<1>(U, g, s, c, form, out); break;
             case 2: acc = plaqforce_dir<2>(U, g, s, c, form, out); break;
@@ -1306,8 +1304,33 @@ __global__ void __launch_bounds__(PF_BS, PfMinBlocks<L, T>::v)
     }
     if (part) {
         const double r = block_sum(acc, sh);
-        if (threadIdx.x == 0) part[(int64_t)blockIdx.y * gridDim.x + blockIdx.x] = r;
+        if (threadIdx.x == 0) part[(int64_t)d * nb + b] = r;
     }
+}
+
+template <class L, typename T>
+__global__ void __launch_bounds__(PF_BS, PfMinBlocks<L, T>::v)
+    k_plaqforce(L U, Geom g, int form, RefOut<T> out, double* part) {
+    __shared__ double sh[32];
+    plaqforce_block<L, T>(blockIdx.x, gridDim.x, blockIdx.y, U, g, form, out, part, sh);
+}
+
+// the FP64 force behind a gate, its grid capped (the Wilson flow's fields that
+// do not take fixed point)
+__global__ void __launch_bounds__(PF_BS)
+    k_plaqforce_gated(FullLinks<double> U, Geom g, RefOut<double> out, unsigned nb, FixGate gt) {
+    __shared__ double sh[32];
+    if (gate_shut(gt)) return;
+    for (unsigned b = blockIdx.x; b < nb; b += gridDim.x)
+        plaqforce_block<FullLinks<double>, double>(b, nb, blockIdx.y, U, g, 0, out, nullptr, sh);
+}
+
+cudaError_t launch_plaquette_force_gated(const FieldRef& U, void* force, const FixGate& gt, cudaStream_t st) {
+    const unsigned nb = (unsigned)plaqforce_blocks(U.g), cap = 8u * (unsigned)device_sms();
+    const FullLinks<double> L{(const double2*)U.links, U.g.V};
+    const RefOut<double> fo{(double2*)force, U.g.V, 4};
+    note_launch(), k_plaqforce_gated<<<dim3(std::min(nb, cap), 4), PF_BS, 0, st>>>(L, U.g, fo, nb, gt);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_plaquette_force(const FieldRef& U, double* part, double* out_S, void* force, int force_form,

@@ -113,24 +113,6 @@ __device__ __forceinline__ FxVS fwd_q_fix(const Geom& g, const PlaneArg& pa, int
     return q;
 }
 
-// the anti-Hermitian q - q^+ as 9 integers of unit 2^-58 (read in units of
-// 2^-61 they are K), in the order of AHFix; q(e) is entry e = 3 a + b
-template <class Q>
-__device__ __forceinline__ void fx_antiherm(Q q, i64 d[9]) {
-    d[0] = 2 * q(0).y;
-    d[1] = 2 * q(4).y;
-    d[2] = 2 * q(8).y;
-    longlong2 u = q(1), l = q(3);
-    d[3] = u.x - l.x;
-    d[4] = u.y + l.y;
-    u = q(2), l = q(6);
-    d[5] = u.x - l.x;
-    d[6] = u.y + l.y;
-    u = q(5), l = q(7);
-    d[7] = u.x - l.x;
-    d[8] = u.y + l.y;
-}
-
 // F = (Q - Q^+)/8 from those integers; fq = Q / q
 __device__ __forceinline__ void fx_field_strength(const i64 d[9], double fq, double f[9]) {
     const double sc = fq * 0x1p-61;

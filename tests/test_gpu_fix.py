@@ -117,3 +117,47 @@ def test_gauge_fixed_time_links_take_fixed_point():
     assert not np.array_equal(g1, g0)
     assert np.linalg.norm(g1 - g0) <= 8e-15 * np.linalg.norm(g0)
     assert abs(e1 - oracle.loop5_energy(u, ALL)) <= 1e-12 * abs(e0)
+
+
+def _flow_step(field, eps, nbytes):
+    f = field.clone()
+    ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+    d = f.descriptor()
+    _lib.call("flue_wflow_step", ctypes.byref(d), eps, _ptr(ws), nbytes, ctypes.c_void_p(0))
+    torch.cuda.synchronize()
+    return f.to_numpy()
+
+
+def _flow_both(u, eps):
+    f = as_field(np.asfortranarray(u))
+    v = f.volume
+    small = _a(36 * v * 16) + _a(36 * v * 8) + _a((v + 127) // 128 * 4 * 8)
+    full = _lib.load().flue_workspace_bytes(_lib.OP_WFLOW, *f.dims, _lib.C128)
+    assert full > small
+    return _flow_step(f, eps, full), _flow_step(f, eps, small)
+
+
+# Entries are of order 1 and rounded to FP64 on both sides (2^-53 each); the
+# FP64 step adds the rounding of its three exponentials: 8 x 2^-53.  eps = 0.1
+# takes |X| past 1/2 (X is halved); 0.13 is past the fixed-point factors' range.
+@pytest.mark.parametrize("dims", [(31, 1, 1, 1), (2, 2, 2, 2), (3, 11, 1, 1), (43, 3, 1, 1), (5, 3, 4, 7), (8, 4, 4, 8)])
+@pytest.mark.parametrize("eps", [0.01, 0.1, 0.13])
+@pytest.mark.parametrize("field_eps", [0.0, 0.3])
+def test_flow_step_against_fp64(dims, eps, field_eps):
+    u = generate.haar_field(dims, 5) if field_eps == 0.0 else generate.random_field(dims, field_eps, 5)
+    a, b = _flow_both(u, eps)
+    assert np.abs(a - b).max() <= 8 * 2.0**-53
+    if eps > 0.12:
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("change", ["scaled", "nan", "cold"])
+def test_flow_stays_in_fp64(change):
+    dims = (7, 5, 4, 3)
+    u = np.array(generate.cold_field(dims) if change == "cold" else generate.random_field(dims, 0.3, 9))
+    if change == "scaled":
+        u[3, 2, 1, 0, 2] *= 1.01
+    elif change == "nan":
+        u[3, 2, 1, 0, 2, 1, 1] = np.nan
+    a, b = _flow_both(u, 0.02)
+    assert np.array_equal(a, b, equal_nan=True)

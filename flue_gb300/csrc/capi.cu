@@ -87,9 +87,9 @@ PlaneSet all_planes() {
 size_t ws_bytes_for(int op, const Geom& g, int prec) {
     switch (op) {
         case FLUE_OP_PLAQUETTE:
-            return a256((size_t)plaquette_slots(g) * 8);
+            return plaquette_ws_bytes(g, prec);
         case FLUE_OP_POLYAKOV:
-            return a256((size_t)polyakov_slots(g) * 16);
+            return polyakov_ws_bytes(g, prec);
         case FLUE_OP_WMUNU:
             return a256((size_t)wloop_slots(g) * 8);
         case FLUE_OP_FMUNU: {
@@ -128,6 +128,8 @@ size_t ws_min_bytes_for(int op, const Geom& g, int prec) {
         return energy_ws_min_bytes(g, prec, ps, false);
     }
     if (op == FLUE_OP_WFLOW) return wflow_ws_min_bytes(g);
+    if (op == FLUE_OP_PLAQUETTE) return plaquette_ws_min_bytes(g);
+    if (op == FLUE_OP_POLYAKOV) return polyakov_ws_min_bytes(g);
     return ws_bytes_for(op, g, prec);
 }
 
@@ -308,7 +310,8 @@ int flue_plaquette(const flue_field* U, int muStart, int muEnd, int nuEnd, doubl
     if (muStart < 1 || muEnd > 4 || nuEnd > 4 || muStart > muEnd + 1 || nuEnd < 1)
         return fail(FLUE_ERR_ARG, "plane range out of 1..4");
     if ((rc = check_ws(FLUE_OP_PLAQUETTE, F, ws_bytes, ws))) return rc;
-    return cuda_status(launch_plaquette(F, muStart - 1, muEnd - 1, nuEnd - 1, (double*)ws, d_sum, (cudaStream_t)stream));
+    return cuda_status(launch_plaquette(F, muStart - 1, muEnd - 1, nuEnd - 1, (double*)ws, ws_bytes, d_sum,
+                                        (cudaStream_t)stream));
 }
 
 size_t flue_wmunu_table_bytes(int nt, int nx, int ny, int nz, int prec, int rmax, int tmax) {
@@ -324,13 +327,13 @@ int flue_wmunu_table(const flue_field* U, int mu, int nu, int rmax, int tmax, do
     if (!d_out) return fail(FLUE_ERR_ARG, "NULL output");
     if (mu < 1 || mu > 4 || nu < 1 || nu > 4) return fail(FLUE_ERR_ARG, "direction out of 1..4");
     if (rmax < 1 || tmax < 1 || rmax > 64 || tmax > 64) return fail(FLUE_ERR_ARG, "rmax, tmax must be 1..64");
-    const size_t need = wmunu_table_ws_bytes(F.g, F.prec, rmax, tmax);
+    const size_t need = wmunu_table_ws_min_bytes(F.g, F.prec, rmax, tmax);
     if (!ws || ws_bytes < need) {
         snprintf(g_detail, sizeof(g_detail), "workspace too small: need %zu bytes, got %zu", need, ws_bytes);
         return FLUE_ERR_WORKSPACE;
     }
     if (((uintptr_t)ws) % 256) return fail(FLUE_ERR_LAYOUT, "workspace must be 256-byte aligned");
-    return cuda_status(launch_wmunu_table(F, mu - 1, nu - 1, rmax, tmax, d_out, ws, (cudaStream_t)stream));
+    return cuda_status(launch_wmunu_table(F, mu - 1, nu - 1, rmax, tmax, d_out, ws, ws_bytes, (cudaStream_t)stream));
 }
 
 int flue_polyakov(const flue_field* U, double* d_sum2, void* ws, size_t ws_bytes, void* stream) {
@@ -339,7 +342,7 @@ int flue_polyakov(const flue_field* U, double* d_sum2, void* ws, size_t ws_bytes
     if (rc) return rc;
     if (!d_sum2) return fail(FLUE_ERR_ARG, "NULL output");
     if ((rc = check_ws(FLUE_OP_POLYAKOV, F, ws_bytes, ws))) return rc;
-    return cuda_status(launch_polyakov(F, (double*)ws, d_sum2, (cudaStream_t)stream));
+    return cuda_status(launch_polyakov(F, (double*)ws, ws_bytes, d_sum2, (cudaStream_t)stream));
 }
 
 int flue_wmunu(const flue_field* U, int tau, int mu, int nu, int nMu, int nNu, double* d_val, void* ws, size_t ws_bytes,

@@ -76,22 +76,33 @@ __device__ __forceinline__ Fx fx_of61(i64 s) {
 __device__ __forceinline__ i64 fx_int60(const Fx& a) { return ((i64)a.h << 31) + a.l; }
 
 // double to Fx, |x| < 2: the 53-bit significand shifted to unit 2^-60
-// (truncated below it), without an FP64 instruction
+// (truncated below it).  In integer instructions: every conversion from or to
+// FP64 runs on the FP64 pipe, 64 cycles a warp.
 __device__ __forceinline__ Fx fx_of(double x) {
     const u32 hw = (u32)__double2hiint(x), lw = (u32)__double2loint(x);
-    const u32 e = (hw >> 20) & 0x7ffu;
-    // significand with its leading 1 at bit 63, then right by 1025 - e
+    // significand with its leading 1 at bit 63, then right by 1025 - exponent
+    // (2 for |x| in [1, 2); the shift clamps at 64)
     const u32 mh = __funnelshift_l(lw, hw, 11) | 0x80000000u, ml = lw << 11;
-    const u32 sh = 1025u - e;  // 2 for |x| in [1, 2); e >= 1025 is refused by link_state
-    u32 xh = sh < 32u ? mh >> sh : 0u;
-    u32 xl = sh < 32u ? __funnelshift_r(ml, mh, sh) : (sh < 64u ? mh >> (sh - 32u) : 0u);
-    const int s = (int)hw >> 31;
-    const i64 m = (i64)(((unsigned long long)xh << 32) | xl);
-    return fx_of61((m ^ (i64)s) - (i64)s);
+    const u32 sh = (0x401fffffu - (hw & 0x7fffffffu)) >> 20;
+    unsigned long long m = ((unsigned long long)mh << 32) | ml;
+    asm("shr.u64 %0, %0, %1;" : "+l"(m) : "r"(sh));
+    const i64 s = (i64)((int)hw >> 31);
+    return fx_of61(((i64)m ^ s) - s);
+}
+// whether fx_of takes x: |x| < 2 (not for infinities and NaN)
+__device__ __forceinline__ bool fx_takes(double x) {
+    return ((u32)__double2hiint(x) & 0x7fffffffu) < 0x40000000u;
 }
 
 using M3F = M3<Fx>;   // a matrix in limbs
 using M3S = M3<i64>;  // a sum of products, unit 2^-58
+
+__device__ __forceinline__ M3F fx_of(const M3<double>& u) {
+    M3F m;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) m.r[k] = fx_of(u.r[k]), m.i[k] = fx_of(u.i[k]);
+    return m;
+}
 
 __device__ __forceinline__ M3S s_zero() {
     M3S m;
@@ -302,9 +313,9 @@ __device__ __forceinline__ void fx_rdot_add(FxVS& S, int a, const FxR& m, const 
     S.i[a] = fx_fold(si);
 }
 
-// Re Tr(op(A) op(B)) as a double; one cross sum per row of A
+// Re Tr(op(A) op(B)), unit 2^-58; one cross sum per row of A
 template <bool DA, bool DB>
-__device__ __forceinline__ double fx_retr(const M3F& A, const M3F& B) {
+__device__ __forceinline__ i64 fx_retr(const M3F& A, const M3F& B) {
     i64 t = 0;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
@@ -317,14 +328,31 @@ __device__ __forceinline__ double fx_retr(const M3F& A, const M3F& B) {
         }
         t += fx_fold(s);
     }
-    return (double)t * 0x1p-58;
+    return t;
+}
+// Re (u . conj v) of two columns, unit 2^-58
+__device__ __forceinline__ i64 fx_rezdot(const FxV& u, const FxV& v) {
+    FxAcc s = {0, FX_CR0};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) fx_mad(s, u.r[k], v.r[k]), fx_mad(s, u.i[k], v.i[k]);
+    return fx_fold(s);
+}
+// Sum over a warp of integers |t| < 2^62 (exact, rounded once to the double):
+// three 22-bit parts by the warp's integer reduction, in place of five FP64
+// additions a lane.
+__device__ __forceinline__ double warp_sum_fix(i64 t) {
+    const u32 m = (1u << 22) - 1;
+    const u32 s0 = __reduce_add_sync(0xffffffffu, (u32)t & m);
+    const u32 s1 = __reduce_add_sync(0xffffffffu, (u32)(t >> 22) & m);
+    const int s2 = __reduce_add_sync(0xffffffffu, (int)(t >> 44));
+    return fma((double)s2, 0x1p44, fma((double)s1, 0x1p22, (double)s0));
 }
 
 // ---------------------------------------------------------------------------
 // the gate between the fixed-point and the FP64 kernels
 // ---------------------------------------------------------------------------
 struct FixGate {
-    u32* p = nullptr;  // [0]: links that are not unitary, [1]: links away from 1
+    u32* p = nullptr;  // [0]: links that are not unitary, [1]: links away from 1, [2]: blocks done
     u32 need = 0;      // open when [0] is 0 and [1] is at least this
     __device__ __forceinline__ bool open() const {
         return *(volatile const u32*)p == 0 && ((volatile const u32*)p)[1] >= need;
@@ -338,13 +366,18 @@ __device__ __forceinline__ bool gate_shut(const FixGate& gt) { return gt.p && gt
 // imaginary parts than fixed point does.  (A quarter: a gauge fixed along one
 // direction has a quarter of its links at 1.)
 constexpr float FIX_FAR2 = 1.f / 256.f;
+constexpr int GATE_WORDS = 3;  // zeroed before the counts
 
-// what the counts of one link are: bit 0 = not unitary (or not finite), bit 1 = away from 1
-__device__ __forceinline__ u32 link_state(const M3<double>& u) {
+// what the counts of one link are: bit 0 = not unitary (or not finite), bit 1 =
+// away from 1; f = fx_of(u)
+__device__ __forceinline__ u32 link_state(const M3<double>& u, const M3F& f) {
     float r[9], i[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) r[k] = (float)u.r[k], i[k] = (float)u.i[k];
     bool ok = true;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        ok = ok && fx_takes(u.r[k]) && fx_takes(u.i[k]);
+        r[k] = (float)f.r[k].h * 0x1p-29f, i[k] = (float)f.i[k].h * 0x1p-29f;
+    }
 #pragma unroll
     for (int a = 0; a < 3; ++a)
 #pragma unroll
@@ -357,9 +390,9 @@ __device__ __forceinline__ u32 link_state(const M3<double>& u) {
                 im = fmaf(i[3 * a + k], r[3 * b + k], im);
                 im = fmaf(-r[3 * a + k], i[3 * b + k], im);
             }
-            // |U U^+ - 1| <= 2^-9 an element (a NaN fails): every norm above is
-            // then within 2% of its unitary value for products of 14 links
-            ok = ok && fabsf(re - (a == b ? 1.f : 0.f)) <= 0x1p-9f && (a == b || fabsf(im) <= 0x1p-9f);
+            // |U U^+ - 1| <= 2^-16 an element (fields stored in single precision
+            // pass): the norm of a product of n links is then within n 2.3e-5 of 1
+            ok = ok && fabsf(re - (a == b ? 1.f : 0.f)) <= 0x1p-16f && (a == b || fabsf(im) <= 0x1p-16f);
         }
     float d2 = 0.f;
 #pragma unroll
@@ -381,16 +414,23 @@ __device__ __forceinline__ void gate_count(const FixGate& gt, u32 st) {
     }
 }
 
+// Whether this block is the last of n to come here (p[2] of the gate counts
+// them); its partial sums and the others' are then visible to it.
+__device__ __forceinline__ bool gate_last_block(const FixGate& gt, u32 n) {
+    __shared__ bool last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(gt.p + 2, 1u) == n - 1;
+    }
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+
 // ---------------------------------------------------------------------------
 // links and intermediates
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ M3F fx_of(const M3<double>& u) {
-    M3F m;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) m.r[k] = fx_of(u.r[k]), m.i[k] = fx_of(u.i[k]);
-    return m;
-}
-
 // One matrix per (plane k, site s): 9 int4 units (h, l of the real and the
 // imaginary part), 144 bytes, in tiles of 32 sites with the units unit-major
 // (unit u of site s at tile + 32 u + s % 32), so that a warp's load of one

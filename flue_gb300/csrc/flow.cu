@@ -337,8 +337,9 @@ __global__ void __launch_bounds__(128) k_flow_links(FullLinks<double> U, Geom g,
     u32 st = 0;
     if (s < g.V) {
         const M3<double> u = U.load(s, (int)blockIdx.y);
-        st = link_state(u);
-        w.store(s, (int)blockIdx.y, fx_of(u));
+        const M3F f = fx_of(u);
+        st = link_state(u, f);
+        w.store(s, (int)blockIdx.y, f);
     }
     gate_count(gt, st);
 }
@@ -527,7 +528,7 @@ cudaError_t launch_wflow_step(void* links, const Geom& g, int prec, double eps, 
     if (prec == PREC_C128 && ws_bytes >= fw.total && eps < 0.12) {
         gt.p = (u32*)(w + fw.gate);
         gt.need = (u32)g.V;  // a quarter of the links
-        cudaError_t e = cudaMemsetAsync(gt.p, 0, 2 * sizeof(u32), st);
+        cudaError_t e = cudaMemsetAsync(gt.p, 0, GATE_WORDS * sizeof(u32), st);
         if (e != cudaSuccess) return e;
         const MatFix w0{(int4*)w, g.V};
         note_launch(), k_flow_links<<<dim3((unsigned)((g.V + 127) / 128), 4), 128, 0, st>>>(

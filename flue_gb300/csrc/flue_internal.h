@@ -66,17 +66,25 @@ int plaquette_slots(const Geom& g);
 int polyakov_slots(const Geom& g);
 int wloop_slots(const Geom& g);
 int meanlink_slots(const Geom& g);
-cudaError_t launch_plaquette(const FieldRef& U, int mu0, int mu1, int nu1, double* part, double* out, cudaStream_t st);
+// *_ws_bytes: what the reduction uses best; *_ws_min_bytes: the least it takes
+// (complex128 fields then run in FP64)
+size_t plaquette_ws_bytes(const Geom& g, int prec);
+size_t plaquette_ws_min_bytes(const Geom& g);
+size_t polyakov_ws_bytes(const Geom& g, int prec);
+size_t polyakov_ws_min_bytes(const Geom& g);
+cudaError_t launch_plaquette(const FieldRef& U, int mu0, int mu1, int nu1, double* part, size_t ws_bytes, double* out,
+                             cudaStream_t st);
 int polyakov_blocks(const Geom& g);
-cudaError_t launch_polyakov(const FieldRef& U, double* part, double* out2, cudaStream_t st);
+cudaError_t launch_polyakov(const FieldRef& U, double* part, size_t ws_bytes, double* out2, cudaStream_t st);
 int wloop_blocks(const Geom& g);
 cudaError_t launch_wloop(const FieldRef& U, int tau, int mu, int nu, int nmu, int nnu, double* part, double* out,
                          cudaStream_t st);
 cudaError_t launch_genericpath(const FieldRef& U, const int* path_host, int npath, const int* coord_host, void* out,
                                cudaStream_t st);
 size_t wmunu_table_ws_bytes(const Geom& g, int prec, int rmax, int tmax);
+size_t wmunu_table_ws_min_bytes(const Geom& g, int prec, int rmax, int tmax);
 cudaError_t launch_wmunu_table(const FieldRef& U, int mu, int nu, int rmax, int tmax, double* out, void* ws,
-                               cudaStream_t st);
+                               size_t ws_bytes, cudaStream_t st);
 int meanlink_blocks(const Geom& g);
 cudaError_t launch_meanlink(const FieldRef& U, const void* G, int g_dtype, double* part, double* out4, cudaStream_t st);
 

@@ -848,7 +848,7 @@ static EnergyWs energy_layout(const Geom& g, int prec, const PlaneArg& pa, bool 
     w.lam = align256(w.kbuf + (with_force ? ah(pa.np) : 0));
     w.part = align256(w.lam + (with_force ? mat(3 * pa.nd) : 0));
     w.gate = align256(w.part + (size_t)pa.np * nbx * sizeof(double));
-    w.gate_bytes = fix ? (2 + (size_t)g.n[0]) * sizeof(u32) : 0;
+    w.gate_bytes = fix ? (GATE_WORDS + (size_t)g.n[0]) * sizeof(u32) : 0;
     w.total = align256(w.gate + w.gate_bytes);
     return w;
 }
@@ -956,9 +956,9 @@ static cudaError_t energy_fwd_part(const L& U, const Geom& g, const Geom& gs, in
         stage_mark(1, st);
         if (w.fix) {
             if (ffits)
-                note_launch(), k_fwd_fix<u32><<<nbx * pa.np, 3 * FIX_BS, 0, st>>>(g, pa, kind, pt, flines, fkb, fout, part, gt.p + 2, ksl, gt);
+                note_launch(), k_fwd_fix<u32><<<nbx * pa.np, 3 * FIX_BS, 0, st>>>(g, pa, kind, pt, flines, fkb, fout, part, gt.p + GATE_WORDS, ksl, gt);
             else
-                note_launch(), k_fwd_fix<int64_t><<<nbx * pa.np, 3 * FIX_BS, 0, st>>>(g, pa, kind, pt, flines, fkb, fout, part, gt.p + 2, ksl, gt);
+                note_launch(), k_fwd_fix<int64_t><<<nbx * pa.np, 3 * FIX_BS, 0, st>>>(g, pa, kind, pt, flines, fkb, fout, part, gt.p + GATE_WORDS, ksl, gt);
         }
         const unsigned nf = nbx * pa.np, gf = gated_grid(w, nf);
         if (fits)
@@ -999,9 +999,9 @@ static cudaError_t energy_fwd_part(const L& U, const Geom& g, const Geom& gs, in
         const unsigned nlf = (unsigned)((g.V + FIX_BS - 1) / FIX_BS) * 3 * pa.nd;
         if (w.fix) {
             if (MatFix::fits32(g.V, 3 * pa.nd) && AHFix::fits32(g.V, pa.np))
-                note_launch(), k_linecot_fix<u32><<<nlf, 3 * FIX_BS, 0, st>>>(g, pa, flines, fkb, flam, gt.p + 2, ksl, gt);
+                note_launch(), k_linecot_fix<u32><<<nlf, 3 * FIX_BS, 0, st>>>(g, pa, flines, fkb, flam, gt.p + GATE_WORDS, ksl, gt);
             else
-                note_launch(), k_linecot_fix<int64_t><<<nlf, 3 * FIX_BS, 0, st>>>(g, pa, flines, fkb, flam, gt.p + 2, ksl, gt);
+                note_launch(), k_linecot_fix<int64_t><<<nlf, 3 * FIX_BS, 0, st>>>(g, pa, flines, fkb, flam, gt.p + GATE_WORDS, ksl, gt);
         }
         if (cfits)
             note_launch(), k_linecot_gated<u32><<<gl, COT_BS, 0, st>>>(g, pa, lines, kb, lam, nl, gt);
@@ -1034,7 +1034,7 @@ static cudaError_t energy_out_part(const Geom& g, const PlaneArg& pa, double vno
         if (w.fix) {
             const MatFix flines{(int4*)(ws + w.lines), g.V}, flam{(int4*)(ws + w.lam), g.V};
             note_launch(), k_linkcot_fix<<<dim3(nb, 4), 128, 0, st>>>(g, pa, flines, flam, scale, form, fo, skip_zero,
-                                                                   gt.p + 2, pa.slot[0] < 0, gt);
+                                                                   gt.p + GATE_WORDS, pa.slot[0] < 0, gt);
             nbg = gated_grid(w, nb);
         }
     }

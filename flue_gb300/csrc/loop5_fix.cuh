@@ -46,8 +46,8 @@ __device__ __forceinline__ u32 line_site_fix(const L& U, const Geom& g, const Ge
     const int64_t s1 = u + (int64_t)wrapd(cd, 1, nd) * sd;
     const int64_t s2 = u + (int64_t)wrapd(cd, 2, nd) * sd;
     const M3<double> ud = U.load(u, d);
-    const u32 st = link_state(ud);
     const M3F u0 = fx_of(ud);
+    const u32 st = link_state(ud, u0);
     lines.store(s, 3 * slot, u0);
     const M3F l2 = fx_mm<false, false>(u0, fx_of(U.load(s1, d)));
     lines.store(s, 3 * slot + 1, l2);

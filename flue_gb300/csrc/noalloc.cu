@@ -11,10 +11,11 @@
 // fixed device array that is part of the library image instead.
 //
 // The array is a file-scope __device__ object of FLUE_NOALLOC_SCRATCH_DOUBLES
-// doubles (8 KiB).  Every GPU on which the library is loaded holds it until
+// doubles (8 KiB) and the 256 bytes of the complex128 fields' fixed-point gate
+// (cleared at the start of every call).  Every GPU on which the library is loaded holds it until
 // the process exits.  It is shared by all calls and keeps the contents of the
-// last call; the kernel writes every slot it later reads, so nothing has to
-// be cleared between calls.  Two calls whose work overlaps on the GPU (for
+// last call; the kernel writes every slot it later reads, so nothing else has
+// to be cleared between calls.  Two calls whose work overlaps on the GPU (for
 // example on two streams at once) race on the array and can both return
 // wrong sums: serialise them.  The array's address is looked up on the first
 // call on each device and kept, so this entry point must not be used across a
@@ -28,7 +29,7 @@
 
 namespace {
 
-static __device__ __align__(256) double g_noalloc_scratch[FLUE_NOALLOC_SCRATCH_DOUBLES];
+static __device__ __align__(256) double g_noalloc_scratch[FLUE_NOALLOC_SCRATCH_DOUBLES + 32];
 
 constexpr int kMaxDevices = 64;
 std::mutex g_noalloc_mtx;
@@ -87,7 +88,8 @@ extern "C" int flue_plaquette_noalloc(const flue_field* U, int muStart, int muEn
         return FLUE_ERR_CUDA;
     }
     return flue::cuda_status(
-        flue::launch_plaquette(F, muStart - 1, muEnd - 1, nuEnd - 1, scratch, d_sum, (cudaStream_t)stream));
+        flue::launch_plaquette(F, muStart - 1, muEnd - 1, nuEnd - 1, scratch,
+                               (FLUE_NOALLOC_SCRATCH_DOUBLES + 32) * sizeof(double), d_sum, (cudaStream_t)stream));
 }
 
 namespace flue {

@@ -7,6 +7,7 @@
 // per block with warp shuffles, and finished by a one-block kernel that adds
 // the block partials in index order, so results are bitwise reproducible for
 // a given lattice size.
+#include <algorithm>
 #include <atomic>
 
 #include "flue_internal.h"
@@ -47,13 +48,16 @@ static int red_cap() {
 // ---------------------------------------------------------------------------
 // reduction finisher
 // ---------------------------------------------------------------------------
-__global__ void k_finish_sums(const double* __restrict__ part, int nparts, double scale, double* __restrict__ out) {
-    __shared__ double sh[32];
-    const double* p = part + (int64_t)blockIdx.x * nparts;
+__device__ __forceinline__ void finish_sum(const double* p, int nparts, double scale, double* out, double* sh) {
     double acc = 0.0;
     for (int i = threadIdx.x; i < nparts; i += blockDim.x) acc += p[i];
     double r = block_sum(acc, sh);
-    if (threadIdx.x == 0) out[blockIdx.x] = scale == 1.0 ? r : r * scale;
+    if (threadIdx.x == 0) *out = scale == 1.0 ? r : r * scale;
+}
+
+__global__ void k_finish_sums(const double* __restrict__ part, int nparts, double scale, double* __restrict__ out) {
+    __shared__ double sh[32];
+    finish_sum(part + (int64_t)blockIdx.x * nparts, nparts, scale, out + blockIdx.x, sh);
 }
 
 cudaError_t launch_finish_sums(const double* partial, int nparts, int nout, double* out, cudaStream_t st, double scale) {
@@ -275,9 +279,8 @@ int plaquette_slots(const Geom& g) { return grid_for(g.V, RED_BS, kMaxRedBlocks)
 #define FLUE_PLAQ_MINB 2
 #endif
 template <class L, typename T>
-__global__ void __launch_bounds__(RED_BS, sizeof(T) == 4 ? FLUE_PLAQ_MINB : 1)
-    k_plaquette(L U, Geom g, int mu0, int mu1, int nu1, double* __restrict__ part) {
-    __shared__ double sh[32];
+__device__ __forceinline__ void plaquette_block(const L& U, const Geom& g, int mu0, int mu1, int nu1,
+                                                double* __restrict__ part, double* sh) {
     double acc = 0.0;
     for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < g.V; s += (int64_t)gridDim.x * blockDim.x) {
         int c[4];
@@ -304,7 +307,126 @@ __global__ void __launch_bounds__(RED_BS, sizeof(T) == 4 ? FLUE_PLAQ_MINB : 1)
     if (threadIdx.x == 0) part[blockIdx.x] = r;
 }
 
-cudaError_t launch_plaquette(const FieldRef& U, int mu0, int mu1, int nu1, double* part, double* out, cudaStream_t st) {
+template <class L, typename T>
+__global__ void __launch_bounds__(RED_BS, sizeof(T) == 4 ? FLUE_PLAQ_MINB : 1)
+    k_plaquette(L U, Geom g, int mu0, int mu1, int nu1, double* __restrict__ part) {
+    __shared__ double sh[32];
+    plaquette_block<L, T>(U, g, mu0, mu1, nu1, part, sh);
+}
+
+// After the fixed-point kernel below: sums its block partials when the gate is
+// open; else computes them in FP64, and the last block to finish sums them.
+__global__ void __launch_bounds__(RED_BS) k_plaquette_finish(FullLinks<double> U, Geom g, int mu0, int mu1, int nu1,
+                                                             double* part, FixGate gt, double* out) {
+    __shared__ double sh[32];
+    if (gt.open()) {
+        if (blockIdx.x) return;
+    } else {
+        plaquette_block<FullLinks<double>, double>(U, g, mu0, mu1, nu1, part, sh);
+        if (!gate_last_block(gt, gridDim.x)) return;
+    }
+    finish_sum(part, gridDim.x, 1.0, out, sh);
+}
+
+// Plaquettes of a complex128 field in fixed point (all planes at 32^3x64 4.7 ->
+// 1.6 ms, half integer multiply-adds, half the conversion of 16 links a site),
+// a thread a site: the site's
+// own links are converted once into shared memory (each of them is in up to
+// three planes), the neighbours' as they are read.  They are counted in the
+// gate on the way: the partial sums stand when the gate turns out open, else
+// k_plaquette_finish replaces them.
+constexpr int PLF_BS = 128;
+constexpr int PLF_SMEM = 36 * PLF_BS * (int)sizeof(int4);  // 73,728: three blocks an SM
+static int plaqfix_blocks(const Geom& g) { return grid_for(g.V, PLF_BS, std::min(3 * device_sms(), kMaxRedBlocks)); }
+
+__device__ __forceinline__ M3F smem_link(const int4* p, int mu) {
+    M3F m;
+#pragma unroll
+    for (int e = 0; e < 9; ++e) {
+        const int4 v = p[(9 * mu + e) * PLF_BS];
+        m.r[e] = {v.x, v.y};
+        m.i[e] = {v.z, v.w};
+    }
+    return m;
+}
+
+__global__ void __launch_bounds__(PLF_BS, 3)
+    k_plaquette_fix(FullLinks<double> U, Geom g, int mu0, int mu1, int nu1, double* __restrict__ part, FixGate gt) {
+    extern __shared__ int4 own_sm[];
+    __shared__ double sh[32];
+    int4* own = own_sm + threadIdx.x;
+    double acc = 0.0;
+    for (int64_t s0 = (int64_t)blockIdx.x * PLF_BS; s0 < g.V; s0 += (int64_t)gridDim.x * PLF_BS) {
+        const int64_t s = s0 + threadIdx.x;
+        const bool live = s < g.V;
+        int c[4];
+        site_coords(g, live ? s : 0, c);
+#pragma unroll 1
+        for (int mu = mu0; mu <= nu1; ++mu) {
+            u32 st = 0;
+            if (live) {
+                const M3<double> u = U.load(s, mu);
+                const M3F f = fx_of(u);
+                st = link_state(u, f);
+#pragma unroll
+                for (int e = 0; e < 9; ++e)
+                    own[(9 * mu + e) * PLF_BS] = make_int4(f.r[e].h, f.r[e].l, f.i[e].h, f.i[e].l);
+            }
+            gate_count(gt, st);
+        }
+        if (!live) continue;
+        int64_t fw[4];
+#pragma unroll
+        for (int d = 0; d < 4; ++d) fw[d] = c[d] + 1 == g.n[d] ? -(int64_t)(g.n[d] - 1) * g.st[d] : g.st[d];
+        i64 t = 0;
+#pragma unroll 1
+        for (int mu = mu0; mu <= mu1; ++mu) {
+            const int64_t sm = s + (mu == 0 ? fw[0] : mu == 1 ? fw[1] : mu == 2 ? fw[2] : fw[3]);
+#pragma unroll 1
+            for (int nu = mu + 1; nu <= nu1; ++nu) {
+                const int64_t sn = s + (nu == 1 ? fw[1] : nu == 2 ? fw[2] : fw[3]);
+                const M3F a = fx_mm<false, false>(smem_link(own, mu), fx_of(U.load(sm, nu)));
+                const M3F b = fx_mm<false, false>(smem_link(own, nu), fx_of(U.load(sn, mu)));
+                t += fx_retr<false, true>(a, b);  // six planes: below 2^63
+            }
+        }
+        acc += (double)t * 0x1p-58;
+    }
+    const double r = block_sum(acc, sh);
+    if (threadIdx.x == 0) part[blockIdx.x] = r;
+}
+
+size_t plaquette_ws_bytes(const Geom& g, int prec) {
+    const size_t red = ((size_t)plaquette_slots(g) * 8 + 255) & ~(size_t)255;
+    return prec == PREC_C128 ? std::max(red, (size_t)kMaxRedBlocks * 8) + 256 : red;
+}
+size_t plaquette_ws_min_bytes(const Geom& g) { return ((size_t)plaquette_slots(g) * 8 + 255) & ~(size_t)255; }
+
+// the gate at the end of a reduction's workspace
+static FixGate red_gate(void* ws, size_t bytes, uint64_t nlinks, cudaStream_t st, cudaError_t* e) {
+    FixGate gt;
+    gt.p = (u32*)((char*)ws + bytes - 256);
+    gt.need = (u32)((nlinks + 3) / 4);
+    *e = cudaMemsetAsync(gt.p, 0, GATE_WORDS * sizeof(u32), st);
+    return gt;
+}
+
+cudaError_t launch_plaquette(const FieldRef& U, int mu0, int mu1, int nu1, double* part, size_t ws_bytes, double* out,
+                             cudaStream_t st) {
+    const size_t fws = plaquette_ws_bytes(U.g, U.prec);
+    if (U.prec == PREC_C128 && ws_bytes >= fws && mu0 <= mu1 && mu0 < nu1) {
+        const FullLinks<double> L{(const double2*)U.links, U.g.V};
+        cudaError_t e;
+        const FixGate gt = red_gate(part, fws, (uint64_t)U.g.V * (nu1 - mu0 + 1), st, &e);
+        if (e != cudaSuccess) return e;
+        const int nb = plaqfix_blocks(U.g);
+        // (the attribute is per function and per device; setting it again is harmless)
+        e = cudaFuncSetAttribute(k_plaquette_fix, cudaFuncAttributeMaxDynamicSharedMemorySize, PLF_SMEM);
+        if (e != cudaSuccess) return e;
+        note_launch(), k_plaquette_fix<<<nb, PLF_BS, PLF_SMEM, st>>>(L, U.g, mu0, mu1, nu1, part, gt);
+        note_launch(), k_plaquette_finish<<<nb, RED_BS, 0, st>>>(L, U.g, mu0, mu1, nu1, part, gt, out);
+        return cudaGetLastError();
+    }
     const int nb = plaquette_blocks(U.g);
     FLUE_DISPATCH_LINKS(U, note_launch(), k_plaquette<decltype(L), T><<<nb, RED_BS, 0, st>>>(L, U.g, mu0, mu1, nu1, part));
     cudaError_t e = cudaGetLastError();
@@ -340,8 +462,7 @@ __device__ __forceinline__ M3<T> shfl_down_m3(const M3<T>& m, int off) {
 }
 
 template <class L, typename T>
-__global__ void __launch_bounds__(RED_BS) k_polyakov(L U, Geom g, double* __restrict__ part) {
-    __shared__ double sh[32];
+__device__ __forceinline__ void polyakov_block(const L& U, const Geom& g, double* __restrict__ part, double* sh) {
     double accr = 0.0, acci = 0.0;
     const int nt = g.n[0];
     const int64_t V3 = g.V / nt;
@@ -382,7 +503,108 @@ __global__ void __launch_bounds__(RED_BS) k_polyakov(L U, Geom g, double* __rest
     if (threadIdx.x == 0) part[gridDim.x + blockIdx.x] = a;
 }
 
-cudaError_t launch_polyakov(const FieldRef& U, double* part, double* out2, cudaStream_t st) {
+template <class L, typename T>
+__global__ void __launch_bounds__(RED_BS) k_polyakov(L U, Geom g, double* __restrict__ part) {
+    __shared__ double sh[32];
+    polyakov_block<L, T>(U, g, part, sh);
+}
+
+// as k_plaquette_finish
+__global__ void __launch_bounds__(RED_BS) k_polyakov_finish(FullLinks<double> U, Geom g, double* part, FixGate gt,
+                                                            double* out2) {
+    __shared__ double sh[32];
+    if (gt.open()) {
+        if (blockIdx.x) return;
+    } else {
+        polyakov_block<FullLinks<double>, double>(U, g, part, sh);
+        if (!gate_last_block(gt, gridDim.x)) return;
+    }
+    finish_sum(part, gridDim.x, 1.0, out2, sh);
+    finish_sum(part + gridDim.x, gridDim.x, 1.0, out2 + 1, sh);
+}
+
+// Polyakov loops of a complex128 field in fixed point: nl lanes a column (a
+// power of two with at least eight links a lane, as far as NT has them), each
+// the ordered product of its run of links, then log2(nl) shuffle levels: few
+// enough for the levels' idle lanes (a lane a link made 6 of 7 products idle
+// work), enough columns in flight for the chip.  32^3x64 0.53 -> 0.24 ms a call.  The links are counted in the
+// gate; k_polyakov_finish replaces the sums when it turns out shut.
+constexpr int POLF_BS = 128;
+static int polyfix_lanes(int nt) {
+    int nl = 1;
+    while (nl < 32 && nt >= 16 * nl) nl *= 2;
+    return nl;
+}
+static int polyfix_blocks(const Geom& g) {
+    return grid_for(g.V / g.n[0], POLF_BS / polyfix_lanes(g.n[0]), kMaxRedBlocks);
+}
+
+__global__ void __launch_bounds__(POLF_BS) k_polyakov_fix(FullLinks<double> U, Geom g, int nl,
+                                                          double* __restrict__ part, FixGate gt) {
+    __shared__ double sh[32];
+    const int nt = g.n[0], lane = threadIdx.x % nl, k = (nt + nl - 1) / nl;
+    const int t0 = min(nt, lane * k), t1 = min(nt, t0 + k);
+    const int64_t V3 = g.V / nt;
+    const int per = POLF_BS / nl;
+    double accr = 0.0, acci = 0.0;
+    for (int64_t r0 = (int64_t)blockIdx.x * per; r0 < V3; r0 += (int64_t)gridDim.x * per) {
+        const int64_t r = r0 + threadIdx.x / nl;
+        const bool live = r < V3;
+        M3F p;
+#pragma unroll
+        for (int e = 0; e < 9; ++e) p.r[e] = {e % 4 == 0 ? 1 << 29 : 0, 0}, p.i[e] = {0, 0};
+#pragma unroll 1
+        for (int j = 0; j < k; ++j) {  // the same count for every lane: gate_count is warp-wide
+            const int t = t0 + j;
+            u32 st = 0;
+            if (live && t < t1) {
+                const M3<double> u = U.load(r * nt + t, 0);
+                const M3F f = fx_of(u);
+                st = link_state(u, f);
+                p = j ? fx_mm<false, false>(p, f) : f;
+            }
+            gate_count(gt, st);
+        }
+#pragma unroll 1
+        for (int off = 1; off < nl; off <<= 1) {
+            M3F q;
+#pragma unroll
+            for (int e = 0; e < 9; ++e) {
+                q.r[e] = {__shfl_down_sync(0xffffffffu, p.r[e].h, off), __shfl_down_sync(0xffffffffu, p.r[e].l, off)};
+                q.i[e] = {__shfl_down_sync(0xffffffffu, p.i[e].h, off), __shfl_down_sync(0xffffffffu, p.i[e].l, off)};
+            }
+            if ((lane & (2 * off - 1)) == 0) p = fx_mm<false, false>(p, q);
+        }
+        if (live && lane == 0) {
+            accr += (double)(fx_int60(p.r[0]) + fx_int60(p.r[4]) + fx_int60(p.r[8])) * 0x1p-60;
+            acci += (double)(fx_int60(p.i[0]) + fx_int60(p.i[4]) + fx_int60(p.i[8])) * 0x1p-60;
+        }
+    }
+    double a = block_sum(accr, sh);
+    if (threadIdx.x == 0) part[blockIdx.x] = a;
+    a = block_sum(acci, sh);
+    if (threadIdx.x == 0) part[gridDim.x + blockIdx.x] = a;
+}
+
+size_t polyakov_ws_min_bytes(const Geom& g) { return ((size_t)polyakov_slots(g) * 16 + 255) & ~(size_t)255; }
+size_t polyakov_ws_bytes(const Geom& g, int prec) {
+    const size_t red = polyakov_ws_min_bytes(g);
+    return prec == PREC_C128 ? std::max(red, (size_t)kMaxRedBlocks * 16) + 256 : red;
+}
+
+cudaError_t launch_polyakov(const FieldRef& U, double* part, size_t ws_bytes, double* out2, cudaStream_t st) {
+    const size_t fws = polyakov_ws_bytes(U.g, U.prec);
+    // (products of up to 4096 links keep their norms within the fixed-point bounds)
+    if (U.prec == PREC_C128 && ws_bytes >= fws && U.g.n[0] <= 4096) {
+        const FullLinks<double> L{(const double2*)U.links, U.g.V};
+        cudaError_t e;
+        const FixGate gt = red_gate(part, fws, (uint64_t)U.g.V, st, &e);
+        if (e != cudaSuccess) return e;
+        const int nbf = polyfix_blocks(U.g);
+        note_launch(), k_polyakov_fix<<<nbf, POLF_BS, 0, st>>>(L, U.g, polyfix_lanes(U.g.n[0]), part, gt);
+        note_launch(), k_polyakov_finish<<<nbf, RED_BS, 0, st>>>(L, U.g, part, gt, out2);
+        return cudaGetLastError();
+    }
     const int nb = U.prec == PREC_C128 ? polyakov_blocks_serial(U.g) : polyakov_blocks(U.g);
     FLUE_DISPATCH_LINKS(U, note_launch(), k_polyakov<decltype(L), T><<<nb, RED_BS, 0, st>>>(L, U.g, part));
     cudaError_t e = cudaGetLastError();
@@ -470,9 +692,8 @@ cudaError_t launch_wloop(const FieldRef& U, int tau, int mu, int nu, int nmu, in
 constexpr int WT_BS = 128;
 
 template <class L, typename T>
-__global__ void k_wt_lines(L U, Geom g, int mu, int nu, int rmax, int tmax, MatAoS<T> lines) {
-    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= g.V) return;
+__device__ __forceinline__ void wt_lines_site(int64_t s, const L& U, const Geom& g, int mu, int nu, int rmax, int tmax,
+                                              const MatAoS<T>& lines) {
     int c[4];
     site_coords(g, s, c);
     for (int pass = 0; pass < 2; ++pass) {
@@ -492,16 +713,21 @@ __global__ void k_wt_lines(L U, Geom g, int mu, int nu, int rmax, int tmax, MatA
     }
 }
 
+template <class L, typename T>
+__global__ void k_wt_lines(L U, Geom g, int mu, int nu, int rmax, int tmax, MatAoS<T> lines) {
+    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (s < g.V) wt_lines_site<L, T>(s, U, g, mu, nu, rmax, tmax, lines);
+}
+
+// block blk of nsb site blocks (of the block's size) x rmax tmax tasks
 template <typename T>
-__global__ void __launch_bounds__(WT_BS) k_wt_loops(Geom g, int mu, int nu, int rmax, int tmax, MatAoS<T> lines,
-                                                    double* __restrict__ part) {
-    __shared__ double sh[32];
+__device__ __forceinline__ void wt_loop_block(unsigned blk, int nsb, const Geom& g, int mu, int nu, int rmax, int tmax,
+                                              const MatAoS<T>& lines, double* __restrict__ part, double* sh) {
     const int nrt = rmax * tmax;
-    const int rt = blockIdx.x % nrt;
-    const int sb = blockIdx.x / nrt;
-    const int nsb = gridDim.x / nrt;
+    const int rt = blk % nrt;
+    const int sb = blk / nrt;
     const int R = rt / tmax + 1, Tl = rt % tmax + 1;
-    const int64_t s = (int64_t)sb * WT_BS + threadIdx.x;
+    const int64_t s = (int64_t)sb * blockDim.x + threadIdx.x;
     double acc = 0.0;
     if (s < g.V) {
         int c[4];
@@ -520,25 +746,148 @@ __global__ void __launch_bounds__(WT_BS) k_wt_loops(Geom g, int mu, int nu, int 
     if (threadIdx.x == 0) part[(int64_t)rt * nsb + sb] = r;
 }
 
+template <typename T>
+__global__ void __launch_bounds__(WT_BS) k_wt_loops(Geom g, int mu, int nu, int rmax, int tmax, MatAoS<T> lines,
+                                                    double* __restrict__ part) {
+    __shared__ double sh[32];
+    wt_loop_block<T>(blockIdx.x, gridDim.x / (rmax * tmax), g, mu, nu, rmax, tmax, lines, part, sh);
+}
+
+// the FP64 kernels of a complex128 field whose gate is shut, their grids capped
+__global__ void __launch_bounds__(WT_BS) k_wt_lines_gated(FullLinks<double> U, Geom g, int mu, int nu, int rmax,
+                                                          int tmax, MatAoS<double> lines, FixGate gt) {
+    if (gate_shut(gt)) return;
+    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < g.V; s += (int64_t)gridDim.x * blockDim.x)
+        wt_lines_site<FullLinks<double>, double>(s, U, g, mu, nu, rmax, tmax, lines);
+}
+__global__ void __launch_bounds__(WT_BS) k_wt_loops_gated(Geom g, int mu, int nu, int rmax, int tmax, int nsb,
+                                                          MatAoS<double> lines, double* __restrict__ part, FixGate gt) {
+    __shared__ double sh[32];
+    if (gate_shut(gt)) return;
+    for (unsigned b = blockIdx.x; b < (unsigned)(nsb * rmax * tmax); b += gridDim.x)
+        wt_loop_block<double>(b, nsb, g, mu, nu, rmax, tmax, lines, part, sh);
+}
+
+// The lines in fixed point, a thread a (site, direction)
+__global__ void __launch_bounds__(WT_BS) k_wt_lines_fix(FullLinks<double> U, Geom g, int mu, int nu, int rmax, int tmax,
+                                                        MatFix lines, FixGate gt) {
+    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int d = blockIdx.y ? nu : mu, n = blockIdx.y ? tmax : rmax, k0 = blockIdx.y ? rmax : 0;
+    u32 st = 0;
+    if (s < g.V) {
+        int c[4];
+        site_coords(g, s, c);
+        int cd = 0, nd = 1;
+        int64_t sd = 1;
+        dir_of(g, c, d, cd, nd, sd);
+        int64_t sw = s;
+        const M3<double> u = U.load(sw, d);
+        M3F p = fx_of(u);
+        st = link_state(u, p);
+        lines.store(s, k0, p);
+#pragma unroll 1
+        for (int k = 1; k < n; ++k) {
+            sw += (cd + 1 == nd) ? -(int64_t)(nd - 1) * sd : sd;
+            cd = (cd + 1 == nd) ? 0 : cd + 1;
+            p = fx_mm<false, false>(p, fx_of(U.load(sw, d)));
+            lines.store(s, k0 + k, p);
+        }
+    }
+    gate_count(gt, st);
+}
+
+// The loops in fixed point, three warps (columns) for 32 sites.  A block has
+// one R and the tmax loops of its sites: column b of A B and of D C and their
+// part of the trace, two matrix-vector products a thread and loop.  32^3x64, 8 x
+// 8 table: FP64 58.8 ms; fixed point 22.6 ms with a barrier a loop, and with one
+// barrier 16.7 ms (128 sites a block, 12 warps an SM), 13.7 (64 sites, 18 warps,
+// 112 registers, spills), 13.4 (32 sites, 15 warps, 136 registers).
+constexpr int WTF_BS = 32, WTF_WARPS = 3 * WTF_BS / 32, WT_MAXT = 64;
+
+template <typename I>
+__global__ void __launch_bounds__(3 * WTF_BS, 5)
+    k_wt_loops_fix(Geom g, int mu, int nu, int rmax, int tmax, MatFix lines, double* __restrict__ part, FixGate gt) {
+    __shared__ double sh[WT_MAXT][WTF_WARPS];  // one barrier for all the loops
+    if (!gt.open()) return;
+    const int R = blockIdx.x % rmax + 1, sb = blockIdx.x / rmax, nsb = gridDim.x / rmax;
+    const int b = threadIdx.x / WTF_BS, w = threadIdx.x >> 5;
+    const int64_t s64 = (int64_t)sb * WTF_BS + threadIdx.x % WTF_BS;
+    const bool live = s64 < g.V;
+    const I s = (I)(live ? s64 : 0);
+    int c[4];
+    site_coords(g, (int64_t)s, c);
+    int cm = 0, nm = 1, cn = 0, nn = 1;
+    int64_t sm = 1, sn = 1;
+    dir_of(g, c, mu, cm, nm, sm);
+    dir_of(g, c, nu, cn, nn, sn);
+    const I sR = (I)((int64_t)s + ((cm + R) % nm - cm) * sm);
+    int ct = cn;
+#pragma unroll 1
+    for (int T = 1; T <= tmax; ++T) {
+        ct = ct + 1 == nn ? 0 : ct + 1;
+        const I sT = (I)((int64_t)s + (ct - cn) * sn);
+        const FxV ab = lines.mul<false>(s, R - 1, lines.col<false>(sR, rmax + T - 1, b));
+        const FxV dc = lines.mul<false>(s, rmax + T - 1, lines.col<false>(sT, R - 1, b));
+        const double r = warp_sum_fix(live ? fx_rezdot(ab, dc) : 0);
+        if ((threadIdx.x & 31) == 0) sh[T - 1][w] = r;
+    }
+    __syncthreads();
+    if (threadIdx.x < tmax) {
+        double sum = 0.0;
+#pragma unroll
+        for (int k = 0; k < WTF_WARPS; ++k) sum += sh[threadIdx.x][k];
+        part[(int64_t)((R - 1) * tmax + threadIdx.x) * nsb + sb] = sum * 0x1p-58;
+    }
+}
+
 // the stored mu- and nu-lines of every length, rounded to 256 bytes
-static size_t wt_lines_bytes(const Geom& g, int prec, int rmax, int tmax) {
-    const size_t b = prec == PREC_C128 ? MatAoS<double>::bytes(g.V, rmax + tmax) : MatAoS<float>::bytes(g.V, rmax + tmax);
+static size_t wt_lines_bytes(const Geom& g, int prec, int rmax, int tmax, bool fix) {
+    size_t b = prec == PREC_C128 ? MatAoS<double>::bytes(g.V, rmax + tmax) : MatAoS<float>::bytes(g.V, rmax + tmax);
+    if (fix) b = std::max(b, MatFix::bytes(g.V, rmax + tmax));
     return (b + 255) & ~(size_t)255;
 }
 
+static size_t wt_ws_bytes(const Geom& g, int prec, int rmax, int tmax, bool fix) {
+    const int bs = fix ? WTF_BS : WT_BS;
+    const size_t nsb = (size_t)((g.V + bs - 1) / bs);
+    const size_t lines = wt_lines_bytes(g, prec, rmax, tmax, fix);
+    return lines + (((size_t)rmax * tmax * nsb * sizeof(double) + 255) & ~(size_t)255) + (fix ? 256 : 0);
+}
 size_t wmunu_table_ws_bytes(const Geom& g, int prec, int rmax, int tmax) {
-    const size_t nsb = (size_t)((g.V + WT_BS - 1) / WT_BS);
-    const size_t lines = wt_lines_bytes(g, prec, rmax, tmax);
-    return lines + (((size_t)rmax * tmax * nsb * sizeof(double) + 255) & ~(size_t)255);
+    return wt_ws_bytes(g, prec, rmax, tmax, prec == PREC_C128);
+}
+size_t wmunu_table_ws_min_bytes(const Geom& g, int prec, int rmax, int tmax) {
+    return wt_ws_bytes(g, prec, rmax, tmax, false);
 }
 
 cudaError_t launch_wmunu_table(const FieldRef& U, int mu, int nu, int rmax, int tmax, double* out, void* ws,
-                               cudaStream_t st) {
+                               size_t ws_bytes, cudaStream_t st) {
     const Geom& g = U.g;
-    const size_t lines_b = wt_lines_bytes(g, U.prec, rmax, tmax);
+    const size_t fws = wmunu_table_ws_bytes(g, U.prec, rmax, tmax);
+    const bool fix = U.prec == PREC_C128 && ws_bytes >= fws;
+    const size_t lines_b = wt_lines_bytes(g, U.prec, rmax, tmax, fix);
     double* part = (double*)((char*)ws + lines_b);
     const unsigned nsb = (unsigned)((g.V + WT_BS - 1) / WT_BS);
     const unsigned nrt = (unsigned)(rmax * tmax);
+    if (fix) {
+        const FullLinks<double> L{(const double2*)U.links, g.V};
+        cudaError_t e;
+        const FixGate gt = red_gate(ws, fws, (uint64_t)g.V * 2, st, &e);
+        if (e != cudaSuccess) return e;
+        const MatFix fl{(int4*)ws, g.V};
+        const MatAoS<double> dl{(double2*)ws, g.V};
+        const unsigned cap = 8u * (unsigned)device_sms(), nsf = (unsigned)((g.V + WTF_BS - 1) / WTF_BS);
+        note_launch(), k_wt_lines_fix<<<dim3(nsb, 2), WT_BS, 0, st>>>(L, g, mu, nu, rmax, tmax, fl, gt);
+        if (MatFix::fits32(g.V, rmax + tmax))
+            note_launch(), k_wt_loops_fix<u32><<<nsf * rmax, 3 * WTF_BS, 0, st>>>(g, mu, nu, rmax, tmax, fl, part, gt);
+        else
+            note_launch(), k_wt_loops_fix<int64_t><<<nsf * rmax, 3 * WTF_BS, 0, st>>>(g, mu, nu, rmax, tmax, fl, part, gt);
+        note_launch(), k_wt_lines_gated<<<std::min(nsb, cap), WT_BS, 0, st>>>(L, g, mu, nu, rmax, tmax, dl, gt);
+        note_launch(), k_wt_loops_gated<<<std::min(nsf * nrt, cap), WTF_BS, 0, st>>>(g, mu, nu, rmax, tmax, (int)nsf, dl,
+                                                                                    part, gt);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        return launch_finish_sums(part, (int)nsf, (int)nrt, out, st, 1.0 / (double)g.V);
+    }
     FLUE_DISPATCH_LINKS(U, {
         MatAoS<T> ln{reinterpret_cast<decltype(MatAoS<T>::p)>(ws), g.V};
         note_launch(), k_wt_lines<decltype(L), T><<<nsb, WT_BS, 0, st>>>(L, g, mu, nu, rmax, tmax, ln);

@@ -161,3 +161,60 @@ def test_flow_stays_in_fp64(change):
         u[3, 2, 1, 0, 2, 1, 1] = np.nan
     a, b = _flow_both(u, 0.02)
     assert np.array_equal(a, b, equal_nan=True)
+
+
+def _loops(field, small):
+    """Plaquette sums of the four kinds of range, the Polyakov sums and a W
+    table on workspaces of the FP64 kernels' size, or of the full size."""
+    L, st = _lib.load(), ctypes.c_void_p(0)
+    nt, nx, ny, nz = field.dims
+    v, d = field.volume, field.descriptor()
+    out = torch.zeros(32, dtype=torch.float64, device="cuda")
+
+    def ws(full, fp64):
+        n = fp64 if small else full
+        assert full > fp64
+        return torch.empty(n, dtype=torch.uint8, device="cuda"), n
+
+    w, n = ws(L.flue_workspace_bytes(_lib.OP_PLAQUETTE, *field.dims, _lib.C128), _a(min(1024, (v + 255) // 256) * 8))
+    for k, r in enumerate(((1, 4, 4), (2, 4, 4), (1, 1, 4), (2, 2, 3), (3, 4, 4))):
+        _lib.call("flue_plaquette", ctypes.byref(d), *r, ctypes.c_void_p(out.data_ptr() + 8 * k), _ptr(w), n, st)
+    w, n = ws(L.flue_workspace_bytes(_lib.OP_POLYAKOV, *field.dims, _lib.C128),
+              _a(min(1024, (v // nt + 7) // 8) * 16))
+    _lib.call("flue_polyakov", ctypes.byref(d), ctypes.c_void_p(out.data_ptr() + 8 * 5), _ptr(w), n, st)
+    nsb = (v + 127) // 128
+    w, n = ws(L.flue_wmunu_table_bytes(*field.dims, _lib.C128, 5, 3), _a(8 * v * 144) + _a(15 * nsb * 8))
+    _lib.call("flue_wmunu_table", ctypes.byref(d), 3, 1, 5, 3, ctypes.c_void_p(out.data_ptr() + 8 * 7), _ptr(w), n, st)
+    torch.cuda.synchronize()
+    return out.cpu().numpy()
+
+
+# Sums over V sites of traces of order 1: each side rounds a trace to 2^-53 and
+# a sum of n terms to at most n 2^-53 of its largest partial sum; 1e-13 a term.
+@pytest.mark.parametrize("dims", [(31, 1, 1, 1), (4, 2, 2, 2), (3, 11, 1, 1), (127, 1, 1, 1), (129, 2, 1, 1), (16, 3, 3, 3),
+                                  (33, 3, 4, 5), (1, 6, 5, 4), (64, 8, 4, 4), (1024, 2, 1, 1)])
+@pytest.mark.parametrize("eps", [0.0, 0.1, 0.4])
+def test_loops_against_fp64(dims, eps):
+    u = generate.haar_field(dims, 5) if eps == 0.0 else generate.random_field(dims, eps, 5)
+    f = as_field(u)
+    a, b = _loops(f, False), _loops(f, True)
+    v = f.volume
+    terms = np.array([6 * v, 3 * v, 3 * v, v, v, v / dims[0], v / dims[0]] + [1.0] * 25)
+    assert (np.abs(a - b) <= 1e-13 * np.maximum(terms, 1)).all()
+
+
+@pytest.mark.parametrize("change", ["scaled", "nan", "cold", "near_cold"])
+def test_loops_stay_in_fp64(change):
+    dims = (18, 5, 4, 3)
+    if change == "cold":
+        u = np.array(generate.cold_field(dims))
+    else:
+        u = np.array(generate.random_field(dims, 1e-3 if change == "near_cold" else 0.3, 9))
+    if change == "scaled":
+        u[3, 2, 1, 0] *= 1.01
+    elif change == "nan":
+        u[3, 2, 1, 0, :, 1, 1] = np.nan
+    f = as_field(np.asfortranarray(u))
+    a, b = _loops(f, False), _loops(f, True)
+    # (the FP64 partial sums are grouped by other blocks)
+    assert np.allclose(a, b, rtol=1e-14, atol=1e-12, equal_nan=True)

@@ -30,12 +30,14 @@
 // sum Re Tr Polyakov, sum Im Tr Polyakov, B^2 (already divided by V), V].
 #include <stdlib.h>
 
+#include <algorithm>
 #include <mutex>
 #include <vector>
 
 #include "../../include/flue_gb300.h"
 #include "flue_internal.h"
 #include "loop5.cuh"
+#include "loop5_fix.cuh"
 
 namespace flue {
 
@@ -84,7 +86,42 @@ struct EnsFlowArgs {
     char* ring;    // kSlots slots of slot_bytes
     size_t slot_bytes;
     PlaneArg pa;   // the B^2 planes
+    int nfields;
+    u32* gates;    // complex128: two words a field (FixGate); NULL otherwise
 };
+
+// complex128: whether field f takes the fixed-point kernel, and whether any
+// field does not (block-wide)
+__device__ __forceinline__ bool ens_open(const EnsFlowArgs& a, int f) {
+    return FixGate{a.gates + 2 * f, (u32)a.fields[f].g.V}.open();
+}
+__device__ __forceinline__ bool ens_any(const EnsFlowArgs& a, bool open) {
+    bool any = false;
+    for (int f = threadIdx.x; f < a.nfields; f += blockDim.x) any = any || ens_open(a, f) == open;
+    return __syncthreads_or(any);
+}
+
+// Counts every field's links in its gate (all four directions: a quarter of
+// them has to be away from 1).  Fields too long for the Polyakov product's
+// bounds count as not unitary.
+__global__ void __launch_bounds__(128) k_ens_gates(EnsFlowArgs a) {
+    for (int f = blockIdx.y; f < a.nfields; f += gridDim.y) {
+        const EnsField fl = a.fields[f];
+        const FullLinks<double> U{(const double2*)fl.links, fl.g.V};
+        const FixGate gt{a.gates + 2 * f, 0};
+        if (fl.g.n[0] > 4096 && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(gt.p, 1u);
+        const int64_t n = 4 * fl.g.V;
+        for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x; i0 < n; i0 += (int64_t)gridDim.x * blockDim.x) {
+            const int64_t i = i0 + threadIdx.x;
+            u32 st = 0;
+            if (i < n) {
+                const M3<double> u = U.load(i % fl.g.V, (int)(i / fl.g.V));
+                st = link_state(u, fx_of(u));
+            }
+            gate_count(gt, st);
+        }
+    }
+}
 
 // Thread 0: wait until *p >= target, at most ~1.7 s; false (and the error
 // flag set) when the wait runs out or another wait already failed.
@@ -156,6 +193,8 @@ __global__ void __launch_bounds__(BS, (FlowMinBlocks<T, BS>::value)) k_ens_flow(
     int* const err = a.ctr + 1;
     int* const lines_done = a.ctr + 2;
     int* const fwd_done = a.ctr + 2 + a.nslabs;
+    // complex128: only the fields that the fixed-point kernel left out
+    if (a.gates && !ens_any(a, false)) return;
     // every task is taken once: at most ntasks + 1 turns per block
     for (int guard = 0; guard <= a.ntasks; ++guard) {
         if (threadIdx.x == 0) cur = atomicAdd(a.ctr, 1);
@@ -163,7 +202,12 @@ __global__ void __launch_bounds__(BS, (FlowMinBlocks<T, BS>::value)) k_ens_flow(
         const int t = cur;
         if (t >= a.ntasks) break;
         const EnsTask tk = a.tasks[t];
-        if (tk.type == TASK_COLS) {
+        const bool mine = !a.gates || !ens_open(a, tk.type == TASK_COLS ? tk.a : a.slabs[tk.a].field);
+        if (!mine) {
+            // the scheduler's counts still move on
+            if (threadIdx.x == 0 && tk.type != TASK_COLS)
+                atomicAdd((tk.type == TASK_LINES ? lines_done : fwd_done) + tk.a, 1);
+        } else if (tk.type == TASK_COLS) {
             const EnsField f = a.fields[tk.a];
             const L U = LinksFrom<L>::make(f.links, f.g.V);
             const int nt = f.g.n[0];
@@ -236,12 +280,157 @@ __global__ void __launch_bounds__(BS, (FlowMinBlocks<T, BS>::value)) k_ens_flow(
     }
 }
 
+// The same scheduler for complex128 fields in fixed point: 384 threads, three
+// (columns) for each of 128 sites.  CH: sites a chunk.
+constexpr int EF_BS = 128;
+template <int CH>
+__global__ void __launch_bounds__(3 * EF_BS) k_ens_flow_fix(EnsFlowArgs a) {
+    __shared__ longlong2 sq[9][EF_BS];
+    __shared__ double sh[32];
+    __shared__ int cur, ok;
+    int* const err = a.ctr + 1;
+    int* const lines_done = a.ctr + 2;
+    int* const fwd_done = a.ctr + 2 + a.nslabs;
+    const int b = threadIdx.x / EF_BS, jt = threadIdx.x % EF_BS;
+    if (!ens_any(a, true)) return;
+    for (int guard = 0; guard <= a.ntasks; ++guard) {
+        if (threadIdx.x == 0) cur = atomicAdd(a.ctr, 1);
+        __syncthreads();
+        const int t = cur;
+        if (t >= a.ntasks) break;
+        const EnsTask tk = a.tasks[t];
+        const int fi = tk.type == TASK_COLS ? tk.a : a.slabs[tk.a].field;
+        const EnsField f = a.fields[fi];
+        const FullLinks<double> U{(const double2*)f.links, f.g.V};
+        const bool mine = ens_open(a, fi);
+        if (!mine) {
+            if (threadIdx.x == 0 && tk.type != TASK_COLS)
+                atomicAdd((tk.type == TASK_LINES ? lines_done : fwd_done) + tk.a, 1);
+        } else if (tk.type == TASK_COLS) {
+            const int nt = f.g.n[0];
+            double v[4] = {0.0, 0.0, 0.0, 0.0};
+            for (int k = threadIdx.x; k < tk.n * nt; k += 3 * EF_BS) {
+                const int64_t s = (int64_t)tk.b * nt + k;
+                int c[4];
+                site_coords(f.g, s, c);
+                i64 tp = 0, sp = 0;
+#pragma unroll 1
+                for (int mu = 0; mu < 3; ++mu) {
+                    const int64_t smu = s + (mu == 0 ? disp(f.g, 0, c[0], 1) : mu == 1 ? disp(f.g, 1, c[1], 1) : disp(f.g, 2, c[2], 1));
+                    const M3F umu = fx_of(U.load(s, mu));
+#pragma unroll 1
+                    for (int nu = mu + 1; nu < 4; ++nu) {
+                        const int64_t snu = s + (nu == 1 ? disp(f.g, 1, c[1], 1) : nu == 2 ? disp(f.g, 2, c[2], 1) : disp(f.g, 3, c[3], 1));
+                        const M3F p = fx_mm<false, false>(umu, fx_of(U.load(smu, nu)));
+                        const M3F q = fx_mm<false, false>(fx_of(U.load(s, nu)), fx_of(U.load(snu, mu)));
+                        const i64 r = fx_retr<false, true>(p, q);
+                        if (mu == 0)
+                            tp += r;
+                        else
+                            sp += r;
+                    }
+                }
+                v[0] += (double)sp * 0x1p-58;
+                v[1] += (double)tp * 0x1p-58;
+            }
+            // eight lanes a column, each its run of links, then three levels
+            // (as k_polyakov_fix); short columns one lane
+            const int nl = nt >= 16 ? 8 : 1, per = 3 * EF_BS / nl, kk = (nt + nl - 1) / nl, lane = threadIdx.x % nl;
+            const int t0 = min(nt, lane * kk), t1 = min(nt, t0 + kk);
+#pragma unroll 1
+            for (int c0 = 0; c0 < tk.n; c0 += per) {
+                const int col = c0 + threadIdx.x / nl;
+                M3F p;
+#pragma unroll
+                for (int e = 0; e < 9; ++e) p.r[e] = {e % 4 == 0 ? 1 << 29 : 0, 0}, p.i[e] = {0, 0};
+                if (col < tk.n) {
+                    const int64_t s0 = (int64_t)(tk.b + col) * nt;
+#pragma unroll 1
+                    for (int tt = t0; tt < t1; ++tt) {
+                        const M3F u = fx_of(U.load(s0 + tt, 0));
+                        p = tt > t0 ? fx_mm<false, false>(p, u) : u;
+                    }
+                }
+#pragma unroll 1
+                for (int off = 1; off < nl; off <<= 1) {
+                    const M3F q = fx_shfl_down(p, off);
+                    if ((lane & (2 * off - 1)) == 0) p = fx_mm<false, false>(p, q);
+                }
+                if (col < tk.n && lane == 0) {
+                    v[2] += (double)(fx_int60(p.r[0]) + fx_int60(p.r[4]) + fx_int60(p.r[8])) * 0x1p-60;
+                    v[3] += (double)(fx_int60(p.i[0]) + fx_int60(p.i[4]) + fx_int60(p.i[8])) * 0x1p-60;
+                }
+            }
+#pragma unroll
+            for (int o = 0; o < 4; ++o) {
+                const double r = block_sum(v[o], sh);
+                if (threadIdx.x == 0) a.part[(int64_t)t * NOBS + o] = r;
+            }
+        } else {
+            const int j = tk.a;
+            const EnsSlab sl = a.slabs[j];
+            const Geom g = make_geom(sl.nts, f.g.n[1], f.g.n[2], f.g.n[3]);
+            const MatFix lines{(int4*)(a.ring + (size_t)(j % kSlots) * a.slot_bytes), g.V};
+            if (tk.type == TASK_LINES) {
+                if (threadIdx.x == 0)
+                    ok = j < kSlots || flow_wait(fwd_done + (j - kSlots), a.slabs[j - kSlots].nchunk, err);
+                __syncthreads();
+#pragma unroll 1
+                for (int h = 0; h < CH && ok; h += EF_BS) {  // a thread a (site, direction)
+                    const int64_t s = (int64_t)tk.b * CH + h + jt;
+                    if (s < g.V) line_site_fix(U, g, f.g, sl.t0, a.pa, lines, s, b);
+                }
+                __syncthreads();
+                if (threadIdx.x == 0) {
+                    __threadfence();
+                    atomicAdd(lines_done + j, 1);
+                }
+            } else {
+                if (threadIdx.x == 0) ok = flow_wait(lines_done + j, sl.nchunk, err);
+                __syncthreads();
+                double e = 0.0;
+#pragma unroll 1
+                for (int h = 0; h < CH && ok; h += EF_BS) {
+                    const int64_t s = (int64_t)tk.b * CH + h + jt;
+#pragma unroll 1
+                    for (int p = 0; p < a.pa.np; ++p) {
+                        if (s < g.V) {
+                            int c[4];
+                            site_coords(g, s, c);
+                            const FxVS q = fwd_q_fix<u32>(g, a.pa, 1, lines, s, c, p, b);
+#pragma unroll
+                            for (int k = 0; k < 3; ++k) sq[3 * k + b][jt] = make_longlong2(q.r[k], q.i[k]);
+                        }
+                        __syncthreads();
+                        if (b == p % 3 && s < g.V) {
+                            i64 d[9];
+                            fx_antiherm([&](int el) { return sq[el][jt]; }, d);
+                            double fv[9];
+                            fx_field_strength(d, FXQ5, fv);
+                            e += ah_norm2(fv);
+                        }
+                        __syncthreads();
+                    }
+                }
+                const double r = block_sum(e, sh);
+                if (threadIdx.x == 0) {
+                    a.part[(int64_t)t * NOBS + 4] = r;
+                    __threadfence();
+                    atomicAdd(fwd_done + j, 1);
+                }
+            }
+        }
+        __syncthreads();
+    }
+}
+
 // out[f*NOBS + o] = sum of the field's task partials in list order (its
 // tasks are ftask[ffirst[f] .. ffirst[f+1])); B^2 divided by V.  When a wait
 // of the scheduler ran out (err != 0) every observable is NaN.
 __global__ void k_ensemble_finish(const double* __restrict__ part, const int* __restrict__ ffirst,
                                   const int* __restrict__ ftask, const EnsField* fields, int nfields,
-                                  const int* __restrict__ err, double* __restrict__ out) {
+                                  const int* __restrict__ err, const int* __restrict__ err2,
+                                  double* __restrict__ out) {
     const int f = blockIdx.x;
     if (f >= nfields) return;
     const int o = threadIdx.x;
@@ -253,7 +442,7 @@ __global__ void k_ensemble_finish(const double* __restrict__ part, const int* __
     double acc = 0.0;
     for (int k = ffirst[f]; k < ffirst[f + 1]; ++k) acc += part[(int64_t)ftask[k] * NOBS + o];
     if (o == 4) acc /= (double)fields[f].g.V;
-    out[f * NOBS + o] = *err ? __longlong_as_double(0x7ff8000000000000LL) : acc;
+    out[f * NOBS + o] = (*err || *err2) ? __longlong_as_double(0x7ff8000000000000LL) : acc;
 }
 
 FLUE_OOB_READER(ensemble)
@@ -271,15 +460,16 @@ struct flue_ensemble {
     int ntasks = 0;
     int nslabs = 0;
     int tile = 0;
-    int grid = 0;
+    int grid = 0, grid_fix = 0;
     int block = 128;
     int with_b2 = 1;
+    bool fix = false;  // complex128 in fixed point where a field's gate allows
     EnsField* d_fields = nullptr;
     EnsSlab* d_slabs = nullptr;
     EnsTask* d_tasks = nullptr;
     int* d_ffirst = nullptr;
     int* d_ftask = nullptr;
-    int* d_ctr = nullptr;  // task counter, error flag, per-slab done counters
+    int* d_ctr = nullptr;  // task counter, error flag, per-slab done counters (complex128: twice, then the gates)
     double* d_part = nullptr;
     char* d_ring = nullptr;
     size_t slot_bytes = 0;
@@ -359,9 +549,30 @@ static PlaneArg b2_plane_arg() {
     return pa;
 }
 
+template <int CH>
+static cudaError_t flow_fix_launch(const flue_ensemble* e, const EnsFlowArgs& args, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)e->grid_fix);
+    cfg.blockDim = dim3(3 * EF_BS);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    note_launch();
+    return cudaLaunchKernelEx(&cfg, k_ens_flow_fix<CH>, args);
+}
+
+// ints of one scheduler's counters, and of all of them (see d_ctr)
+static size_t ctr_ints(const flue_ensemble* e) { return 2 + 2 * (size_t)e->nslabs; }
+static size_t ctr_total(const flue_ensemble* e) {
+    return e->fix ? 2 * ctr_ints(e) + 2 * (size_t)e->nfields : ctr_ints(e);
+}
+
 static cudaError_t ens_launch(flue_ensemble* e, double* d_out, cudaStream_t st) {
     if (e->pipeline) return ens_launch_pipeline(e, d_out, st);
-    cudaError_t r = cudaMemsetAsync(e->d_ctr, 0, sizeof(int) * (2 + 2 * (size_t)e->nslabs), st);
+    cudaError_t r = cudaMemsetAsync(e->d_ctr, 0, sizeof(int) * ctr_total(e), st);
     if (r != cudaSuccess) return r;
     EnsFlowArgs args;
     args.fields = e->d_fields;
@@ -374,10 +585,24 @@ static cudaError_t ens_launch(flue_ensemble* e, double* d_out, cudaStream_t st) 
     args.ring = e->d_ring;
     args.slot_bytes = e->slot_bytes;
     args.pa = b2_plane_arg();
+    args.nfields = e->nfields;
+    args.gates = nullptr;
+    const int* err2 = e->d_ctr + 1;
+    if (e->fix) {
+        // fields that pass the gate in fixed point, then the others in FP64 (a
+        // scheduler and counters of their own; nothing to do, as a rule)
+        args.gates = (u32*)(e->d_ctr + 2 * ctr_ints(e));
+        const unsigned gy = (unsigned)std::min(e->nfields, 65535);
+        note_launch(), k_ens_gates<<<dim3(std::max(1u, 4096u / gy), gy), 128, 0, st>>>(args);
+        r = e->block == 256 ? flow_fix_launch<256>(e, args, st) : flow_fix_launch<128>(e, args, st);
+        if (r != cudaSuccess) return r;
+        args.ctr = e->d_ctr + ctr_ints(e);
+        err2 = args.ctr + 1;
+    }
     r = e->block == 256 ? flow_dispatch<256>(e, args, st) : flow_dispatch<128>(e, args, st);
     if (r != cudaSuccess) return r;
     note_launch(), k_ensemble_finish<<<e->nfields, 32, 0, st>>>(e->d_part, e->d_ffirst, e->d_ftask, e->d_fields,
-                                                               e->nfields, e->d_ctr + 1, d_out);
+                                                               e->nfields, e->d_ctr + 1, err2, d_out);
     return cudaGetLastError();
 }
 
@@ -443,6 +668,7 @@ int flue_ensemble_create(flue_ensemble** out, const flue_field* fields, int nfie
     std::vector<EnsTask> tasks;
     std::vector<std::vector<int>> per_field(nfields);
     int64_t max_slab = 1;
+    bool fix = prec == FLUE_C128;
     if (!pipeline) {
         for (int f = 0; f < nfields && with_b2; ++f) {
             const Geom& g = hf[f].g;
@@ -457,6 +683,7 @@ int flue_ensemble_create(flue_ensemble** out, const flue_field* fields, int nfie
                 // the forward reads a slab's lines with 32-bit offsets
                 if (!(prec == FLUE_C128 ? MatAoS<double>::fits32(vs, 9) : MatAoS<float>::fits32(vs, 9)))
                     return FLUE_ERR_SHAPE;
+                fix = fix && MatFix::fits32(vs, 9);
                 if (vs > max_slab) max_slab = vs;
                 slabs.push_back({f, t0, n, (int)((vs + block - 1) / block)});
             }
@@ -497,6 +724,7 @@ int flue_ensemble_create(flue_ensemble** out, const flue_field* fields, int nfie
     e->tile = tile_cols;
     e->block = block;
     e->with_b2 = with_b2 ? 1 : 0;
+    e->fix = fix;
     cudaError_t r = cudaSuccess;
     if (pipeline) {
         e->pipeline = 1;
@@ -522,7 +750,20 @@ int flue_ensemble_create(flue_ensemble** out, const flue_field* fields, int nfie
         e->grid = nsm * (blocks_per_sm < occ ? blocks_per_sm : occ);
         e->ntasks = (int)tasks.size();
         e->nslabs = (int)slabs.size();
-        e->slot_bytes = (prec == PREC_C128 ? MatAoS<double>::bytes(max_slab, 9) : MatAoS<float>::bytes(max_slab, 9));
+        if (fix) {
+            int n = 0;
+            const cudaError_t ro =
+                block == 256 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_ens_flow_fix<256>, 3 * EF_BS, 0)
+                             : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_ens_flow_fix<128>, 3 * EF_BS, 0);
+            if (ro != cudaSuccess || n < 1) {
+                ens_free(e);
+                cudaGetLastError();
+                return FLUE_ERR_CUDA;
+            }
+            e->grid_fix = nsm * n;
+        }
+        e->slot_bytes = prec == PREC_C128 ? std::max(MatAoS<double>::bytes(max_slab, 9), MatFix::bytes(max_slab, 9))
+                                          : MatAoS<float>::bytes(max_slab, 9);
         e->slot_bytes = (e->slot_bytes + 255) & ~(size_t)255;
         if ((r = cudaMalloc(&e->d_ring, kSlots * e->slot_bytes)) != cudaSuccess) {
             ens_free(e);
@@ -535,7 +776,7 @@ int flue_ensemble_create(flue_ensemble** out, const flue_field* fields, int nfie
         (r = cudaMalloc(&e->d_tasks, sizeof(EnsTask) * tasks.size())) != cudaSuccess ||
         (r = cudaMalloc(&e->d_ffirst, sizeof(int) * (nfields + 1))) != cudaSuccess ||
         (r = cudaMalloc(&e->d_ftask, sizeof(int) * ftask.size())) != cudaSuccess ||
-        (r = cudaMalloc(&e->d_ctr, sizeof(int) * (2 + 2 * slabs.size()))) != cudaSuccess ||
+        (r = cudaMalloc(&e->d_ctr, sizeof(int) * (2 * (2 + 2 * slabs.size()) + 2 * (size_t)nfields))) != cudaSuccess ||
         (r = cudaMalloc(&e->d_part, sizeof(double) * NOBS * tasks.size())) != cudaSuccess) {
         ens_free(e);
         cudaGetLastError();

@@ -104,6 +104,15 @@ __device__ __forceinline__ M3F fx_of(const M3<double>& u) {
     return m;
 }
 
+__device__ __forceinline__ M3F fx_shfl_down(const M3F& p, int off) {
+    M3F q;
+#pragma unroll
+    for (int e = 0; e < 9; ++e) {
+        q.r[e] = {__shfl_down_sync(0xffffffffu, p.r[e].h, off), __shfl_down_sync(0xffffffffu, p.r[e].l, off)};
+        q.i[e] = {__shfl_down_sync(0xffffffffu, p.i[e].h, off), __shfl_down_sync(0xffffffffu, p.i[e].l, off)};
+    }
+    return q;
+}
 __device__ __forceinline__ M3S s_zero() {
     M3S m;
 #pragma unroll

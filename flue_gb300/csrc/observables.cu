@@ -567,12 +567,7 @@ __global__ void __launch_bounds__(POLF_BS) k_polyakov_fix(FullLinks<double> U, G
         }
 #pragma unroll 1
         for (int off = 1; off < nl; off <<= 1) {
-            M3F q;
-#pragma unroll
-            for (int e = 0; e < 9; ++e) {
-                q.r[e] = {__shfl_down_sync(0xffffffffu, p.r[e].h, off), __shfl_down_sync(0xffffffffu, p.r[e].l, off)};
-                q.i[e] = {__shfl_down_sync(0xffffffffu, p.i[e].h, off), __shfl_down_sync(0xffffffffu, p.i[e].l, off)};
-            }
+            const M3F q = fx_shfl_down(p, off);
             if ((lane & (2 * off - 1)) == 0) p = fx_mm<false, false>(p, q);
         }
         if (live && lane == 0) {

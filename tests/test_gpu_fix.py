@@ -218,3 +218,30 @@ def test_loops_stay_in_fp64(change):
     a, b = _loops(f, False), _loops(f, True)
     # (the FP64 partial sums are grouped by other blocks)
     assert np.allclose(a, b, rtol=1e-14, atol=1e-12, equal_nan=True)
+
+
+def test_ensemble_mixes_fixed_point_and_fp64_fields():
+    """Fields that pass the gate and fields that do not, in one evaluation: each
+    as the device entry points give it (their own gate decides the same way);
+    tolerance as in test_loops_against_fp64 and test_fixed_point_against_fp64."""
+    from flue_gb300 import gluonCalc as G
+    from flue_gb300.ensemble import Ensemble
+
+    us = [np.array(generate.random_field(d, 0.3, 3 + i)) for i, d in enumerate([(8, 6, 5, 4), (5, 3, 3, 3), (17, 4, 4, 4)])]
+    us.append(np.array(generate.cold_field((6, 4, 4, 4))))
+    bad = us[0].copy()
+    bad[3, 2, 1, 0] *= 1.01
+    us.append(bad)
+    fields = [as_field(np.asfortranarray(u)) for u in us]
+    for block in (128, 256):
+        e = Ensemble(fields, block=block)
+        rows = e.run()
+        assert np.array_equal(rows, e.run())
+        for f, r in zip(fields, rows):
+            v = f.volume
+            assert abs(r[0] - G.plaquette(f, 2, 4, 4)[0]) <= 1e-13 * 3 * v
+            assert abs(r[1] - G.plaquette(f, 1, 1, 4)[0]) <= 1e-13 * 3 * v
+            re, _, _, im = G.polyakov(f, return_imag=True)
+            assert abs(r[2] - re) <= 1e-13 * v and abs(r[3] - im) <= 1e-13 * v
+            b2 = G.magnetic(f)
+            assert abs(r[4] - b2) <= 1e-14 * abs(b2) + 1e-28

@@ -247,7 +247,7 @@ def magnetic_force(data, prec="c128", form="lie", nt=None, nx=None, ny=None, nz=
     forms = {"lie": _lib.FORCE_LIE, "euclid": _lib.FORCE_EUCLID}
     if prec not in precs or form not in forms:
         raise ValueError("prec must be c128/c64/r12 and form lie/euclid")
-    grad = np.zeros_like(a, order="F")
+    grad = np.empty_like(a, order="F")  # every element is written
     b = ctypes.c_double()
     _call("flue_magnetic_force_c", _p(a), _lib.C128, *dims, precs[prec], forms[form], ctypes.byref(b), _p(grad))
     return b.value, grad

@@ -363,6 +363,30 @@ struct FullLinks {
     }
 };
 
+// The same field through 32-bit byte offsets, for fields below 4 GB (fits): a
+// matrix takes one offset register and nine plane addresses that are the same
+// for the whole grid (uniform registers), in place of nine 64-bit additions.
+struct FullLinks32 {
+    const char* __restrict__ p;
+    uint32_t V;
+    __device__ __forceinline__ M3<float> load(uint32_t s, int mu) const {
+        M3<float> m;
+        if (!FLUE_INB(s < V && mu >= 0 && mu < 4)) return m_zero<float>();
+        const uint32_t off = (s + V * (uint32_t)mu) * 8u;
+        const size_t st = (size_t)V * 32;
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+                const float2 v = __ldg(reinterpret_cast<const float2*>(p + st * (a + 3 * b) + off));
+                m.r[3 * a + b] = v.x;
+                m.i[3 * a + b] = v.y;
+            }
+        return m;
+    }
+    static bool fits(int64_t V) { return (uint64_t)V * 32 < (1ull << 32); }
+};
+
 __device__ __forceinline__ void reconstruct_row2(M3<float>& m) {
     // row2 = conj(row0 x row1)  (vector_product of FixSU3Matrix)
 #pragma unroll

@@ -99,13 +99,16 @@ __device__ __forceinline__ int64_t patch_site(const Geom& g, const PatchArg& pt,
            (int64_t)(bo * pt.po + io) * sto;
 }
 
+#ifndef FLUE_PATCH_MAXTW
+#define FLUE_PATCH_MAXTW 32
+#endif
 #ifndef FLUE_PATCH_MIN_TW
 #define FLUE_PATCH_MIN_TW 8
 #endif
 static PatchArg make_patch(const Geom& g, const PlaneArg& pa, int bs) {
     PatchArg pt{0, 1, 1, 1};
     int tw = 1;
-    while (tw < 32 && g.n[0] % (2 * tw) == 0 && tw * 2 <= bs) tw *= 2;
+    while (tw < FLUE_PATCH_MAXTW && g.n[0] % (2 * tw) == 0 && tw * 2 <= bs) tw *= 2;
     const int P = bs / tw;
     int pm = 1;
     while (pm < 4 && pm * pm * 4 <= P) pm *= 2;  // pm = pn <= 4
@@ -175,6 +178,9 @@ __global__ void __launch_bounds__(128) k_lines_gated(FullLinks<double> U, Geom g
 #ifndef FLUE_FWD_MINB
 #define FLUE_FWD_MINB 3
 #endif
+#ifndef FLUE_CLV_MINB
+#define FLUE_CLV_MINB 4
+#endif
 #ifndef FLUE_COT_BS
 #define FLUE_COT_BS 128
 #endif
@@ -198,10 +204,15 @@ constexpr int FWD_BS = FLUE_FWD_BS;
 // next), so registers count for more than warps: B^2 force at 32^3x64 63.0 ms;
 // 64 sites with two blocks an SM 63.2, three (112 registers, spills) 67.6; 32
 // sites with four or five blocks 69.2, 69.9.
-#ifndef FLUE_FIX_BS
-#define FLUE_FIX_BS 128
-#endif
-constexpr int FIX_BS = FLUE_FIX_BS;
+constexpr int FIX_BS = 128;
+// The forward of a small lattice takes blocks of 32 sites, four an SM: below
+// three blocks of 128 sites an SM the last wave is mostly empty.  B^2 at 8^3x16
+// 194 -> 173 us, 10^3x16 254 -> 241, 12^3x24 497 -> 511 (so not there); two
+// halves of the leaves on twice the threads gave 182, 272, 502.
+constexpr int FIX_BS_SMALL = 32;
+static int fix_fwd_block(int64_t V, int planes) {
+    return (V + FIX_BS - 1) / FIX_BS * planes < 3 * device_sms() ? FIX_BS_SMALL : FIX_BS;
+}
 
 // site j of the bs sites of block b of the forward's grid, plane p = b % np
 // (planes of the same site block run in adjacent blocks: L2 reuse)
@@ -254,16 +265,16 @@ __global__ void __launch_bounds__(FWD_BS)
 // warps (columns) for every 32 sites.  32^3x64, three planes: FP64 pipe 81.1 ms,
 // fixed point with a thread a site 20.7 ms (240 registers, 8 warps an SM), with
 // a thread a column 19.0 ms.
-template <typename I>
-__global__ void __launch_bounds__(3 * FIX_BS)
+template <int BS, typename I>
+__global__ void __launch_bounds__(3 * BS, FIX_BS / BS)
     k_fwd_fix(Geom g, PlaneArg pa, int kind, PatchArg pt, MatFix lines, AHFix kout, RefOut<double> fout, double* part,
               u32* kmax, bool kslice, FixGate gt) {
-    __shared__ longlong2 sq[9][FIX_BS];
+    __shared__ longlong2 sq[9][BS];
     __shared__ double sh[32];
     if (!gt.open()) return;
     const int p = blockIdx.x % pa.np;
-    const int b = threadIdx.x / FIX_BS, j = threadIdx.x % FIX_BS;
-    const int64_t s = fwd_site(g, pa, pt, blockIdx.x, p, j, FIX_BS);
+    const int b = threadIdx.x / BS, j = threadIdx.x % BS;
+    const int64_t s = fwd_site(g, pa, pt, blockIdx.x, p, j, BS);
     double e = 0.0;
     int c[4];
     if (s < g.V) {
@@ -273,7 +284,7 @@ __global__ void __launch_bounds__(3 * FIX_BS)
         for (int a = 0; a < 3; ++a) sq[3 * a + b][j] = make_longlong2(q.r[a], q.i[a]);
     }
     __syncthreads();
-    if (b == 0 && s < g.V) {
+    if (threadIdx.x < BS && s < g.V) {
         i64 d[9];
         fx_antiherm([&](int el) { return sq[el][j]; }, d);
         double f[9];
@@ -840,7 +851,7 @@ static EnergyWs energy_layout(const Geom& g, int prec, const PlaneArg& pa, bool 
     };
     EnergyWs w;
     w.fix = fix;
-    const int fbs = fix ? FIX_BS : FWD_BS;
+    const int fbs = fix ? FIX_BS_SMALL : FWD_BS;  // (any SM count's choice of fix_fwd_block fits)
     const int nbx = (int)((g.V + fbs - 1) / fbs);
     w.lines = 0;
     // daggered line copies only when the line cotangents run
@@ -935,7 +946,7 @@ static cudaError_t energy_fwd_part(const L& U, const Geom& g, const Geom& gs, in
     MatAoS<T> lam{reinterpret_cast<decltype(MatAoS<T>::p)>(ws + w.lam), g.V};
     double* part = out_E ? (double*)(ws + w.part) : nullptr;
     const unsigned nbl = (unsigned)((g.V + 127) / 128);
-    const int fbs = w.fix ? FIX_BS : FWD_BS;  // sites a block of the forward covers
+    const int fbs = w.fix ? fix_fwd_block(g.V, pa.np) : FWD_BS;  // sites a block of the forward covers
     const unsigned nbx = (unsigned)((g.V + fbs - 1) / fbs);
     const unsigned nbc = (unsigned)((g.V + COT_BS - 1) / COT_BS);
     const PatchArg pt = FLUE_FWD_PATCH ? make_patch(g, pa, fbs) : PatchArg{};
@@ -955,10 +966,16 @@ static cudaError_t energy_fwd_part(const L& U, const Geom& g, const Geom& gs, in
         note_launch(), k_lines_gated<<<dim3(gated_grid(w, nbl), pa.nd), 128, 0, st>>>(U, g, gs, t0, pa, lines, gt);
         stage_mark(1, st);
         if (w.fix) {
-            if (ffits)
-                note_launch(), k_fwd_fix<u32><<<nbx * pa.np, 3 * FIX_BS, 0, st>>>(g, pa, kind, pt, flines, fkb, fout, part, gt.p + GATE_WORDS, ksl, gt);
+            auto fwd = [&](auto kernel) {
+                note_launch(), kernel<<<nbx * pa.np, 3 * fbs, 0, st>>>(g, pa, kind, pt, flines, fkb, fout, part,
+                                                                       gt.p + GATE_WORDS, ksl, gt);
+            };
+            if (fbs == FIX_BS_SMALL)
+                fwd(k_fwd_fix<FIX_BS_SMALL, u32>);  // (a small lattice fits 32-bit offsets)
+            else if (ffits)
+                fwd(k_fwd_fix<FIX_BS, u32>);
             else
-                note_launch(), k_fwd_fix<int64_t><<<nbx * pa.np, 3 * FIX_BS, 0, st>>>(g, pa, kind, pt, flines, fkb, fout, part, gt.p + GATE_WORDS, ksl, gt);
+                fwd(k_fwd_fix<FIX_BS, int64_t>);
         }
         const unsigned nf = nbx * pa.np, gf = gated_grid(w, nf);
         if (fits)
@@ -996,12 +1013,15 @@ static cudaError_t energy_fwd_part(const L& U, const Geom& g, const Geom& gs, in
         const MatFix flines{(int4*)(ws + w.lines), g.V}, flam{(int4*)(ws + w.lam), g.V};
         const AHFix fkb{(longlong2*)(ws + w.kbuf), g.V};
         const unsigned nl = nbc * 3 * pa.nd, gl = gated_grid(w, nl);
-        const unsigned nlf = (unsigned)((g.V + FIX_BS - 1) / FIX_BS) * 3 * pa.nd;
         if (w.fix) {
+            const unsigned nlf = (unsigned)((g.V + FIX_BS - 1) / FIX_BS) * 3 * pa.nd;
+            auto cot = [&](auto kernel) {
+                note_launch(), kernel<<<nlf, 3 * FIX_BS, 0, st>>>(g, pa, flines, fkb, flam, gt.p + GATE_WORDS, ksl, gt);
+            };
             if (MatFix::fits32(g.V, 3 * pa.nd) && AHFix::fits32(g.V, pa.np))
-                note_launch(), k_linecot_fix<u32><<<nlf, 3 * FIX_BS, 0, st>>>(g, pa, flines, fkb, flam, gt.p + GATE_WORDS, ksl, gt);
+                cot(k_linecot_fix<u32>);
             else
-                note_launch(), k_linecot_fix<int64_t><<<nlf, 3 * FIX_BS, 0, st>>>(g, pa, flines, fkb, flam, gt.p + GATE_WORDS, ksl, gt);
+                cot(k_linecot_fix<int64_t>);
         }
         if (cfits)
             note_launch(), k_linecot_gated<u32><<<gl, COT_BS, 0, st>>>(g, pa, lines, kb, lam, nl, gt);
@@ -1216,6 +1236,26 @@ cudaError_t launch_energy_slabs(const FieldRef& U, const PlaneSet& ps, double* o
     return e;
 }
 
+// Clover of an FP32 field straight from the links (its only lines are links):
+// 24^3x48 c64 117 us through the line buffers.
+template <class L, typename I>
+__global__ void __launch_bounds__(FWD_BS, FLUE_CLV_MINB) k_clover(L U, Geom g, int mu, int nu, RefOut<float> fout) {
+    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= g.V) return;
+    int c[4];
+    site_coords(g, s, c);
+    int mM = 0, mP = 0, nM = 0, nP = 0;
+#pragma unroll
+    for (int d = 0; d < 4; ++d) {
+        const int up = wrapd(c[d], 1, g.n[d]) * (int)g.st[d], dn = wrapd(c[d], -1, g.n[d]) * (int)g.st[d];
+        if (d == mu) mP = up, mM = dn;
+        if (d == nu) nP = up, nM = dn;
+    }
+    const M3<float> q = four_leaves<float>([&](int site) { return U.load((I)site, mu); },
+                                           [&](int site) { return U.load((I)site, nu); }, (int)s, mM, mP, nM, nP);
+    fout.store(s, 0, transp(ah_quarter(q)));
+}
+
 // F_munu of one plane: kind 0 = clover (cloverLoopMuNuCoord), 1 = 5-loop
 // (Loop5MuNuCoord).  Output (NT,NX,NY,NZ,3,3) in the field's compute dtype.
 cudaError_t launch_fmunu(const FieldRef& U, int kind, int mu, int nu, void* out, void* ws, size_t ws_bytes,
@@ -1227,6 +1267,17 @@ cudaError_t launch_fmunu(const FieldRef& U, int kind, int mu, int nu, void* out,
     const PlaneArg pa = make_planes(ps);
     const EnergyWs w = energy_layout_for(U.g, U.prec, pa, false, ws_bytes);
     if (ws_bytes < w.total) return cudaErrorInvalidValue;
+    if (kind == 0 && U.prec != PREC_C128) {
+        const RefOut<float> fo{(float2*)out, U.g.V, 1};
+        const unsigned nb = (unsigned)((U.g.V + FWD_BS - 1) / FWD_BS);
+        if (U.prec == PREC_R12)
+            note_launch(), k_clover<R12Links, int64_t><<<nb, FWD_BS, 0, st>>>(R12Links{(const float4*)U.links, U.g.V}, U.g, mu, nu, fo);
+        else if (FullLinks32::fits(U.g.V))
+            note_launch(), k_clover<FullLinks32, u32><<<nb, FWD_BS, 0, st>>>(FullLinks32{(const char*)U.links, (u32)U.g.V}, U.g, mu, nu, fo);
+        else
+            note_launch(), k_clover<FullLinks<float>, int64_t><<<nb, FWD_BS, 0, st>>>(FullLinks<float>{(const float2*)U.links, U.g.V}, U.g, mu, nu, fo);
+        return cudaGetLastError();
+    }
     FLUE_DISPATCH_LINKS(U, {
         using C2 = typename V2<T>::type;
         RefOut<T> fo{(C2*)out, U.g.V, 1};

@@ -226,6 +226,36 @@ __device__ __forceinline__ M3<T> fwd_q5(const MatAoS<T>& lines, const Ctx& cx) {
     return q;
 }
 
+// Sum of the four leaves of shape (a, b) at site s0: mL(i, j) / nL(i, j) the
+// mu- and nu-line of that length at offset (i a mu + j b nu).  Dagger patterns
+// are fixed at compile time (lines are loaded undaggered):
+//   TR = Lm(0,0) Ln(a,0) Lm(0,b)^+ Ln(0,0)^+
+//   TL = Ln(0,0) Lm(-a,b)^+ Ln(-a,0)^+ Lm(-a,0)
+//   BL = Lm(-a,0)^+ Ln(-a,-b)^+ Lm(-a,-b) Ln(0,-b)
+//   BR = Ln(0,-b)^+ Lm(0,-b) Ln(a,-b) Lm(0,0)^+
+// Lm(0,0), Ln(0,0), Lm(-a,0), Ln(0,-b) serve two leaves each.  mM, mP, nM, nP:
+// the steps of -a mu, a mu, -b nu, b nu.
+template <typename T, class Lm, class Ln>
+__device__ __forceinline__ M3<T> four_leaves(Lm lm, Ln ln, int s0, int mM, int mP, int nM, int nP) {
+    const M3<T> m00 = lm(s0);
+    const M3<T> n00 = ln(s0);
+    M3<T> t = mm<false, false>(m00, ln(s0 + mP));
+    t = mm<false, true>(t, lm(s0 + nP));
+    M3<T> w = mm<false, true>(t, n00);  // TR
+    const M3<T> ma0 = lm(s0 + mM);
+    t = mm<false, true>(n00, lm(s0 + mM + nP));
+    t = mm<false, true>(t, ln(s0 + mM));
+    mac<false, false>(w, t, ma0);  // TL
+    const M3<T> n0b = ln(s0 + nM);
+    t = mm<true, true>(ma0, ln(s0 + mM + nM));
+    t = mm<false, false>(t, lm(s0 + mM + nM));
+    mac<false, false>(w, t, n0b);  // BL
+    t = mm<true, false>(n0b, lm(s0 + nM));
+    t = mm<false, false>(t, ln(s0 + mP + nM));
+    mac<false, true>(w, t, m00);  // BR
+    return w;
+}
+
 template <typename T, typename I>
 __device__ __forceinline__ M3<T> fwd_q(const Geom& g, const PlaneArg& pa, int kind, const MatAoS<T>& lines, int64_t s,
                                        const int c[4], int p) {
@@ -245,14 +275,6 @@ __device__ __forceinline__ M3<T> fwd_q(const Geom& g, const PlaneArg& pa, int ki
     const Shape* shp = kind == 1 ? c_shapes5 : c_shapes1;
     const int nsh = kind == 1 ? 7 : 1;
     M3<T> q = m_zero<T>();
-    // Per shape the four quadrant leaves, with their dagger patterns fixed
-    // at compile time (lines are loaded undaggered; L(i,j) = line at
-    // offset (i mu + j nu)):
-    //   TR = Lm(0,0) Ln(a,0) Lm(0,b)^+ Ln(0,0)^+
-    //   TL = Ln(0,0) Lm(-a,b)^+ Ln(-a,0)^+ Lm(-a,0)
-    //   BL = Lm(-a,0)^+ Ln(-a,-b)^+ Lm(-a,-b) Ln(0,-b)
-    //   BR = Ln(0,-b)^+ Lm(0,-b) Ln(a,-b) Lm(0,0)^+
-    // Lm(0,0), Ln(0,0), Lm(-a,0), Ln(0,-b) serve two leaves each.
 #pragma unroll 1
     for (int k = 0; k < nsh; ++k) {
         const int a = shp[k].a, b = shp[k].b;
@@ -263,26 +285,8 @@ __device__ __forceinline__ M3<T> fwd_q(const Geom& g, const PlaneArg& pa, int ki
         const int s0 = (int)cx.s, stm = (int)cx.stm, stn = (int)cx.stn;
         const int mM = wrapd(cx.cm, -a, cx.nm) * stm, mP = wrapd(cx.cm, a, cx.nm) * stm;
         const int nM = wrapd(cx.cn, -b, cx.nn) * stn, nP = wrapd(cx.cn, b, cx.nn) * stn;
-        auto ld = [&](int site, int k) { return ldm(lines, (I)site, k); };
-        M3<T> w;
-        {
-            const M3<T> m00 = ld(s0, km);
-            const M3<T> n00 = ld(s0, kn);
-            M3<T> t = mm<false, false>(m00, ld(s0 + mP, kn));
-            t = mm<false, true>(t, ld(s0 + nP, km));
-            w = mm<false, true>(t, n00);  // TR
-            const M3<T> ma0 = ld(s0 + mM, km);
-            t = mm<false, true>(n00, ld(s0 + mM + nP, km));
-            t = mm<false, true>(t, ld(s0 + mM, kn));
-            mac<false, false>(w, t, ma0);  // TL
-            const M3<T> n0b = ld(s0 + nM, kn);
-            t = mm<true, true>(ma0, ld(s0 + mM + nM, kn));
-            t = mm<false, false>(t, ld(s0 + mM + nM, km));
-            mac<false, false>(w, t, n0b);  // BL
-            t = mm<true, false>(n0b, ld(s0 + nM, km));
-            t = mm<false, false>(t, ld(s0 + mP + nM, kn));
-            mac<false, true>(w, t, m00);  // BR
-        }
+        const M3<T> w = four_leaves<T>([&](int site) { return ldm(lines, (I)site, km); },
+                                       [&](int site) { return ldm(lines, (I)site, kn); }, s0, mM, mP, nM, nP);
         m_axpy(q, (T)shp[k].c, w);
     }
     return q;

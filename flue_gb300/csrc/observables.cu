@@ -287,7 +287,7 @@ __device__ __forceinline__ void plaquette_block(const L& U, const Geom& g, int m
         site_coords(g, s, c);
         int64_t sp[4];  // s + mu for every direction (compile-time indices only)
 #pragma unroll
-        for (int d = 0; d < 4; ++d) sp[d] = s + disp(g, d, c[d], 1);
+        for (int d = 0; d < 4; ++d) sp[d] = s + (c[d] + 1 == g.n[d] ? -(int64_t)(g.n[d] - 1) * g.st[d] : g.st[d]);
         // the six planes unrolled; the requested range selects them at run time
 #pragma unroll
         for (int mu = 0; mu < 3; ++mu) {
@@ -428,7 +428,12 @@ cudaError_t launch_plaquette(const FieldRef& U, int mu0, int mu1, int nu1, doubl
         return cudaGetLastError();
     }
     const int nb = plaquette_blocks(U.g);
-    FLUE_DISPATCH_LINKS(U, note_launch(), k_plaquette<decltype(L), T><<<nb, RED_BS, 0, st>>>(L, U.g, mu0, mu1, nu1, part));
+    if (U.prec == PREC_C64 && FullLinks32::fits(U.g.V)) {
+        const FullLinks32 L{(const char*)U.links, (uint32_t)U.g.V};
+        note_launch(), k_plaquette<FullLinks32, float><<<nb, RED_BS, 0, st>>>(L, U.g, mu0, mu1, nu1, part);
+    } else {
+        FLUE_DISPATCH_LINKS(U, note_launch(), k_plaquette<decltype(L), T><<<nb, RED_BS, 0, st>>>(L, U.g, mu0, mu1, nu1, part));
+    }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     return launch_finish_sums(part, nb, 1, out, st);

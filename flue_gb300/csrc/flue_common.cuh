@@ -851,14 +851,14 @@ __host__ __device__ inline Geom make_geom(int nt, int nx, int ny, int nz) {
     return g;
 }
 
+// (a lattice has fewer than 2^31 sites: 32-bit divisions)
 __device__ __forceinline__ void site_coords(const Geom& g, int64_t s, int c[4]) {
-    int64_t r = s;
-    c[0] = (int)(r % g.n[0]);
-    r /= g.n[0];
-    c[1] = (int)(r % g.n[1]);
-    r /= g.n[1];
-    c[2] = (int)(r % g.n[2]);
-    c[3] = (int)(r / g.n[2]);
+    const uint32_t n0 = (uint32_t)g.n[0], n1 = (uint32_t)g.n[1], n2 = (uint32_t)g.n[2];
+    const uint32_t r = (uint32_t)s, r1 = r / n0, r2 = r1 / n1, r3 = r2 / n2;
+    c[0] = (int)(r - r1 * n0);
+    c[1] = (int)(r1 - r2 * n1);
+    c[2] = (int)(r2 - r3 * n2);
+    c[3] = (int)r3;
 }
 
 // Site offset of a displacement by k (any sign, |k| <= 4*n) along mu from a

@@ -76,7 +76,7 @@ struct PatchArg {
     int tw, pm, pn, po;
 };
 
-__device__ __forceinline__ int64_t patch_site(const Geom& g, const PatchArg& pt, int pmu, int pnu, int64_t r, int tid) {
+__device__ __forceinline__ int64_t patch_site(const Geom& g, const PatchArg& pt, int pmu, int pnu, unsigned r, int tid) {
     int nm = 1, nn = 1;
     int64_t stm = 0, stn = 0, sto = 0;
     const int od = 6 - pmu - pnu;
@@ -86,7 +86,7 @@ __device__ __forceinline__ int64_t patch_site(const Geom& g, const PatchArg& pt,
         if (d == pnu) nn = g.n[d], stn = g.st[d];
         if (d == od) sto = g.st[d];
     }
-    const int ntc = g.n[0] / pt.tw, nbm = nm / pt.pm, nbn = nn / pt.pn;
+    const unsigned ntc = g.n[0] / pt.tw, nbm = nm / pt.pm, nbn = nn / pt.pn;
     const int tc = (int)(r % ntc);
     r /= ntc;
     const int bi = (int)(r % nbm);

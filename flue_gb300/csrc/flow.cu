@@ -541,28 +541,48 @@ __global__ void __launch_bounds__(3 * FF_BS)
 #pragma unroll
         for (int e = 0; e < 9; ++e) x[e] = fx_of61((((i64)x[e].h << 32) + 2 * (i64)x[e].l) >> 1);
     }
+    // exp(X) U - U = [sum Y^j / (2j)!] U + X [sum Y^j / (2j+1)!] U, Y = X^2
+    // Hermitian: half the matrix-vector products of the plain series
+    Fx y[9];
+    fx_ah_square(x, y);
     FxV u = w.col<false>(s, mu, b);
 #pragma unroll 1
     for (int rep = 0; rep < reps; ++rep) {
-        FxAcc sr[3], si[3];
-#pragma unroll
-        for (int a = 0; a < 3; ++a) sr[a] = si[a] = {FX_HI0, FX_CR0};
-        FxV t = u;
-        float bnd = 1.f;
-#pragma unroll 1
-        for (int k = 1; k <= FLOW_TERMS; ++k) {
-            bnd *= nrm / (float)k;
-            if (!(bnd > 0x1p-62f)) break;
-            const FxVP tp = fx_prep<false>(t);
-#pragma unroll
-            for (int a = 0; a < 3; ++a) fx_rdot_limbs(t.r[a], t.i[a], ah_row(x, a), tp);
-#pragma unroll
-            for (int a = 0; a < 3; ++a) fx_mad(sr[a], t.r[a], c_flow_fact.f[k]), fx_mad(si[a], t.i[a], c_flow_fact.f[k]);
-        }
+        FxAcc er[3], ei[3], odr[3], odi[3];
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            u.r[a] = fx_const60(fx_int60(u.r[a]) + fx_int60(fx_limbs(sr[a])));
-            u.i[a] = fx_const60(fx_int60(u.i[a]) + fx_int60(fx_limbs(si[a])));
+            er[a] = ei[a] = {0, FX_CR0};
+            odr[a] = odi[a] = {FX_HI0, FX_CR0};
+            fx_mad(odr[a], u.r[a], c_flow_fact.f[1]), fx_mad(odi[a], u.i[a], c_flow_fact.f[1]);
+        }
+        FxV t = u;
+        float bnd = nrm;
+#pragma unroll 1
+        for (int k = 2; k < FLOW_TERMS; k += 2) {
+            bnd *= nrm / (float)k;  // |X|^k / k!
+            if (!(bnd > 0x1p-60f)) break;
+            const FxVP tp = fx_prep<false>(t);
+#pragma unroll
+            for (int a = 0; a < 3; ++a) fx_rdot_limbs(t.r[a], t.i[a], he_row(y, a), tp);
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                fx_mad(er[a], t.r[a], c_flow_fact.f[k]), fx_mad(ei[a], t.i[a], c_flow_fact.f[k]);
+                fx_mad(odr[a], t.r[a], c_flow_fact.f[k + 1]), fx_mad(odi[a], t.i[a], c_flow_fact.f[k + 1]);
+            }
+            bnd *= nrm / (float)(k + 1);
+        }
+        FxVS d;
+        FxV o;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            d.r[a] = fx_fold(er[a]), d.i[a] = fx_fold(ei[a]);
+            o.r[a] = fx_limbs(odr[a]), o.i[a] = fx_limbs(odi[a]);
+        }
+        fx_add_kv(d, x, fx_prep<false>(o));
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            u.r[a] = fx_const60(fx_int60(u.r[a]) + 4 * d.r[a]);
+            u.i[a] = fx_const60(fx_int60(u.i[a]) + 4 * d.i[a]);
         }
     }
     if (!live) return;

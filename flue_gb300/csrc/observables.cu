@@ -50,7 +50,16 @@ static int red_cap() {
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void finish_sum(const double* p, int nparts, double scale, double* out, double* sh) {
     double acc = 0.0;
-    for (int i = threadIdx.x; i < nparts; i += blockDim.x) acc += p[i];
+    int i = threadIdx.x;
+    const int st = blockDim.x;
+    for (; i + 7 * st < nparts; i += 8 * st) {  // eight loads in flight, added in order
+        double v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = __ldcg(p + i + k * st);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc += v[k];
+    }
+    for (; i < nparts; i += st) acc += p[i];
     double r = block_sum(acc, sh);
     if (threadIdx.x == 0) *out = scale == 1.0 ? r : r * scale;
 }

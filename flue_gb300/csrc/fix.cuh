@@ -37,7 +37,7 @@ struct Fx {
     int h, l;
 };
 
-// an accumulator: hi of unit 2^-58, cr of unit 2^-90
+// an accumulator: hi of unit 2^-58, cr of unit 2^-89
 struct FxAcc {
     i64 hi, cr;
 };

@@ -369,7 +369,8 @@ __global__ void k_wflow_update(double2* links, Geom g, const double2* force, AHP
 // direction a pass over the lattice read 3.1 GB from DRAM for 0.6 GB of links).
 // Bound by instruction issue (71%, three quarters of it FMA).  32^3x64, a step:
 // force and update apart 4.9 ms, fused 3.42 (128 registers; 168: 3.49, 96:
-// 3.48), with 32-bit offsets 3.22, with expm1_ah 3.03.
+// 3.48), with 32-bit offsets 3.22, with expm1_ah 3.03,
+// with the site coordinates by 32-bit divisions 2.94.
 template <int STAGE, class L, typename I>
 __global__ void __launch_bounds__(128, 4)
     k_flow_stage32(L U, Geom g, AHPlanes<float> bbuf, float eps, float2* out) {

@@ -99,16 +99,13 @@ __device__ __forceinline__ int64_t patch_site(const Geom& g, const PatchArg& pt,
            (int64_t)(bo * pt.po + io) * sto;
 }
 
-#ifndef FLUE_PATCH_MAXTW
-#define FLUE_PATCH_MAXTW 32
-#endif
 #ifndef FLUE_PATCH_MIN_TW
 #define FLUE_PATCH_MIN_TW 8
 #endif
 static PatchArg make_patch(const Geom& g, const PlaneArg& pa, int bs) {
     PatchArg pt{0, 1, 1, 1};
     int tw = 1;
-    while (tw < FLUE_PATCH_MAXTW && g.n[0] % (2 * tw) == 0 && tw * 2 <= bs) tw *= 2;
+    while (tw < 32 && g.n[0] % (2 * tw) == 0 && tw * 2 <= bs) tw *= 2;
     const int P = bs / tw;
     int pm = 1;
     while (pm < 4 && pm * pm * 4 <= P) pm *= 2;  // pm = pn <= 4
@@ -177,9 +174,6 @@ __global__ void __launch_bounds__(128) k_lines_gated(FullLinks<double> U, Geom g
 #endif
 #ifndef FLUE_FWD_MINB
 #define FLUE_FWD_MINB 3
-#endif
-#ifndef FLUE_CLV_MINB
-#define FLUE_CLV_MINB 4
 #endif
 #ifndef FLUE_COT_BS
 #define FLUE_COT_BS 128
@@ -854,7 +848,7 @@ static EnergyWs energy_layout(const Geom& g, int prec, const PlaneArg& pa, bool 
     const int fbs = fix ? FIX_BS_SMALL : FWD_BS;  // (any SM count's choice of fix_fwd_block fits)
     const int nbx = (int)((g.V + fbs - 1) / fbs);
     w.lines = 0;
-    // daggered line copies only when the line cotangents run
+    // K and the line cotangents only with a gradient
     w.kbuf = align256(w.lines + mat(3 * pa.nd));
     w.lam = align256(w.kbuf + (with_force ? ah(pa.np) : 0));
     w.part = align256(w.lam + (with_force ? mat(3 * pa.nd) : 0));
@@ -1236,10 +1230,14 @@ cudaError_t launch_energy_slabs(const FieldRef& U, const PlaneSet& ps, double* o
     return e;
 }
 
-// Clover of an FP32 field straight from the links (its only lines are links):
-// 24^3x48 c64 117 us through the line buffers.
+// Clover of an FP32 field straight from the links: its only lines are links, so
+// the line buffers were a copy of them, written and read back.  12 products from
+// eight links a site, the links' second and third reads from L2: latency and L2
+// bound.  24^3x48 c64 117 us through the line buffers, 60 us so, at 4 blocks of
+// 128 an SM (128 registers; with 3 the latency is less hidden, with 5 it spills).
+constexpr int CLOVER_MINB = 4;
 template <class L, typename I>
-__global__ void __launch_bounds__(FWD_BS, FLUE_CLV_MINB) k_clover(L U, Geom g, int mu, int nu, RefOut<float> fout) {
+__global__ void __launch_bounds__(FWD_BS, CLOVER_MINB) k_clover(L U, Geom g, int mu, int nu, RefOut<float> fout) {
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= g.V) return;
     int c[4];

@@ -282,8 +282,10 @@ int plaquette_slots(const Geom& g) { return grid_for(g.V, RED_BS, kMaxRedBlocks)
 
 // FP32: at most 128 registers (two 256-thread blocks per SM): measured on
 // GB300 at 32^3x64, all planes, c64 0.53 -> 0.36 ms per call against the
-// unbounded unrolled kernel's 0.45 ms; FP64 keeps its registers (bound by the
-// FP64 pipe, it spills under the cap)
+// unbounded unrolled kernel's 0.45 ms; then with 32-bit offsets (FullLinks32)
+// and site coordinates 48^3x96 1.60 -> 1.26 ms (HBM floor 0.83 ms; bound by
+// the latency of its L2 reads).  FP64 keeps its registers (bound by the FP64
+// pipe, it spills under the cap)
 #ifndef FLUE_PLAQ_MINB
 #define FLUE_PLAQ_MINB 2
 #endif
@@ -810,7 +812,8 @@ __global__ void __launch_bounds__(WT_BS) k_wt_lines_fix(FullLinks<double> U, Geo
 // part of the trace, two matrix-vector products a thread and loop.  32^3x64, 8 x
 // 8 table: FP64 58.8 ms; fixed point 22.6 ms with a barrier a loop, and with one
 // barrier 16.7 ms (128 sites a block, 12 warps an SM), 13.7 (64 sites, 18 warps,
-// 112 registers, spills), 13.4 (32 sites, 15 warps, 136 registers).
+// 112 registers, spills), 13.4 (32 sites, 15 warps, 136 registers); 13.2 with the
+// site coordinates by 32-bit divisions.
 constexpr int WTF_BS = 32, WTF_WARPS = 3 * WTF_BS / 32, WT_MAXT = 64;
 
 template <typename I>

@@ -80,8 +80,8 @@ class Ensemble:
         elif tile is None:
             # measured on GB300, 96 fields of 16^3x32 .. 32^3x64: 16 columns per
             # plaquette / Polyakov task, 128 threads, 3 blocks per SM: 111 ms
-            # FP32 (c64) and 3.46 s FP64 per evaluation (pipeline mode 115 ms,
-            # 3.48 s); 4 columns 118 ms, 2 blocks per SM 146 ms
+            # FP32 (c64) and 0.75 s complex128 per evaluation (pipeline mode
+            # 110 ms, 0.76 s); 4 columns 118 ms, 2 blocks per SM 146 ms
             tile = 16
         self.config = (int(tile), int(block), int(blocks_per_sm))
         self._descs = (_lib.FlueField * len(fields))(*[f.descriptor() for f in fields])

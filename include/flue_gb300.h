@@ -96,7 +96,9 @@ const char *flue_strerror(int status);
 int flue_abi_version(void);
 /* bytes of a device field of this size and precision */
 int64_t flue_field_bytes(int nt, int nx, int ny, int nz, int prec);
-/* scratch bytes needed by the device entry point `op` (0 if none) */
+/* scratch bytes of the device entry point `op` (0 if none).  For FLUE_C128
+ * fields it has room for the scratch of the fixed-point kernels; a buffer
+ * sized for the FP64 kernels alone is accepted too and takes those (slower). */
 size_t flue_workspace_bytes(int op, int nt, int nx, int ny, int nz, int prec);
 /* Detail text of the last failure on the calling thread. */
 const char *flue_last_error_detail(void);
@@ -109,7 +111,7 @@ const char *flue_last_error_detail(void);
 int flue_stage_timing(int enable);
 int flue_stage_times(double *ms, int max_stages, int *n_stages);
 /* Number of GPU kernels this library has launched in this process (all
- * devices; a replayed ensemble graph counts its two kernels).  For launch
+ * devices; a replayed ensemble graph counts the kernels it holds).  For launch
  * accounting by benchmarks and tests; no reference counterpart. */
 uint64_t flue_kernel_launches(void);
 /* Bounds-checked build only (compiled with -DFLUE_BOUNDS_CHECK=1): the number
@@ -229,7 +231,9 @@ int flue_gluon_propagator(const flue_field *U, double xi, int mu_start, double *
  * task list from an atomic counter: the 5-loop lines of a chunk of a time
  * slab, the line-based B^2 of a chunk (each waiting, with a bounded wait,
  * for its slab's lines), and plaquettes / Polyakov loops of tile_cols time
- * columns; a finisher sums each field's partials in list order.  A wait that
+ * columns; a finisher sums each field's partials in list order.  (complex128
+ * fields: a gate kernel over their links, this launch in fixed point for the
+ * unitary ones, a second one in FP64 for the others.)  A wait that
  * runs out (not met in a healthy run) makes every output NaN.  One
  * ensemble's evaluations share its counters and line buffers: they must not
  * overlap on the GPU (run them in order on one stream).

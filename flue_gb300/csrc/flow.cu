@@ -223,22 +223,52 @@ __device__ __forceinline__ void ff_addprod(FF& s, float a, float b) {
     s.lo = __fadd_rn(s.lo, __fadd_rn(err, e));
 }
 
+// The same for sums that stay within +-2, in 4 instructions a product instead of
+// 10: hi carries 6 + the sum, so it keeps one exponent, every step of it is a
+// multiple of 2^-21 and known exactly, and what the step rounded off the product
+// (below 2^-22) goes to lo.  The sum is good to about 2^-43, far below the one
+// rounding of the result.  54 products a link: RK3 step at 32^3x64 2.94 -> 2.76 ms.
+struct FB {
+    float hi, lo;
+    __device__ __forceinline__ float sum() const { return __fadd_rn(__fsub_rn(hi, 6.0f), lo); }
+    __device__ __forceinline__ float minus1() const { return __fadd_rn(__fsub_rn(hi, 7.0f), lo); }
+};
+__device__ __forceinline__ void fb_addprod(FB& s, float a, float b) {
+    const float t = __fmaf_rn(a, b, s.hi);
+    const float q = __fsub_rn(t, s.hi);
+    s.hi = t;
+    s.lo = __fadd_rn(s.lo, __fmaf_rn(a, b, -q));
+}
+
+struct SumFF : FF {
+    __device__ __forceinline__ SumFF() : FF{0.f, 0.f} {}
+    __device__ __forceinline__ void add(float a, float b) { ff_addprod(*this, a, b); }
+    __device__ __forceinline__ float sum() const { return hi + lo; }
+    __device__ __forceinline__ float minus1() const { return __fadd_rn(__fsub_rn(hi, 1.0f), lo); }
+};
+struct SumFB : FB {
+    __device__ __forceinline__ SumFB() : FB{6.f, 0.f} {}
+    __device__ __forceinline__ void add(float a, float b) { fb_addprod(*this, a, b); }
+};
+
 // Row r of length^2 1 + delta -> r (1 + c), c = (1 + delta)^-1/2 - 1, with
-// delta from the float-float sum so the row is rounded once.
-__device__ __forceinline__ void ff_normalise(float r[3], float i[3]) {
-    FF n{0.f, 0.f};
+// delta from the compensated sum so the row is rounded once; returns delta.
+template <class Sum>
+__device__ __forceinline__ float ff_normalise(float r[3], float i[3]) {
+    Sum n;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        ff_addprod(n, r[c], r[c]);
-        ff_addprod(n, i[c], i[c]);
+        n.add(r[c], r[c]);
+        n.add(i[c], i[c]);
     }
-    const float d = __fadd_rn(__fsub_rn(n.hi, 1.0f), n.lo);
+    const float d = n.minus1();
     const float c = fabsf(d) < 1e-3f ? d * (-0.5f + d * (0.375f - 0.3125f * d)) : rsqrtf(1.0f + d) - 1.0f;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         r[k] = fmaf(c, r[k], r[k]);
         i[k] = fmaf(c, i[k], i[k]);
     }
+    return d;
 }
 
 // FixSU3Matrix (row 0 normalised, row 1 orthogonalised and normalised,
@@ -248,55 +278,68 @@ __device__ __forceinline__ void ff_normalise(float r[3], float i[3]) {
 // FP32 would.  With plain FP32 sums the flowed B^2 of a 32^3x64 field
 // drifted from the FP64 flow by 2.8e-6 (relative) after 200 steps of 0.01;
 // with these sums by 9.5e-8, the same as with FixSU3Matrix in FP64.
-__device__ __forceinline__ void fix_su3_rows_f32(float r[3][3], float i[3][3]) {
-    ff_normalise(r[0], i[0]);
-    FF dr{0.f, 0.f}, di{0.f, 0.f};
+// False when a row's length^2 was not within 1/2 of 1 (or not a number): with
+// SumFB the result is then not to be used.
+template <class Sum>
+__device__ __forceinline__ bool fix_su3_rows_f32(float r[3][3], float i[3][3]) {
+    const float n1 = r[1][0] * r[1][0] + i[1][0] * i[1][0] + r[1][1] * r[1][1] + i[1][1] * i[1][1] +
+                     r[1][2] * r[1][2] + i[1][2] * i[1][2];
+    const float d0 = ff_normalise<Sum>(r[0], i[0]);
+    Sum dr, di;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        ff_addprod(dr, r[0][c], r[1][c]);
-        ff_addprod(dr, i[0][c], i[1][c]);
-        ff_addprod(di, r[0][c], i[1][c]);
-        ff_addprod(di, -i[0][c], r[1][c]);
+        dr.add(r[0][c], r[1][c]);
+        dr.add(i[0][c], i[1][c]);
+        di.add(r[0][c], i[1][c]);
+        di.add(-i[0][c], r[1][c]);
     }
-    const float ovr = dr.hi + dr.lo, ovi = di.hi + di.lo;
+    const float ovr = dr.sum(), ovi = di.sum();
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         r[1][c] -= r[0][c] * ovr - i[0][c] * ovi;
         i[1][c] -= r[0][c] * ovi + i[0][c] * ovr;
     }
-    ff_normalise(r[1], i[1]);
+    const float d1 = ff_normalise<Sum>(r[1], i[1]);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         const int j = (c + 1) % 3, k = (c + 2) % 3;
-        FF re{0.f, 0.f}, im{0.f, 0.f};
-        ff_addprod(re, r[0][j], r[1][k]);
-        ff_addprod(re, -i[0][j], i[1][k]);
-        ff_addprod(re, -r[0][k], r[1][j]);
-        ff_addprod(re, i[0][k], i[1][j]);
-        ff_addprod(im, r[0][j], i[1][k]);
-        ff_addprod(im, i[0][j], r[1][k]);
-        ff_addprod(im, -r[0][k], i[1][j]);
-        ff_addprod(im, -i[0][k], r[1][j]);
-        r[2][c] = re.hi + re.lo;
-        i[2][c] = -(im.hi + im.lo);
+        Sum re, im;
+        re.add(r[0][j], r[1][k]);
+        re.add(-i[0][j], i[1][k]);
+        re.add(-r[0][k], r[1][j]);
+        re.add(i[0][k], i[1][j]);
+        im.add(r[0][j], i[1][k]);
+        im.add(i[0][j], r[1][k]);
+        im.add(-r[0][k], i[1][j]);
+        im.add(-i[0][k], r[1][j]);
+        r[2][c] = re.sum();
+        i[2][c] = -im.sum();
     }
-    ff_normalise(r[2], i[2]);
+    ff_normalise<Sum>(r[2], i[2]);
+    return fabsf(d0) < 0.5f && fabsf(d1) < 0.5f && fabsf(n1 - 1.0f) < 0.5f;
 }
 
 template <typename W>
 __device__ __forceinline__ void reunitarise(M3<W>& w) {
     W r[3][3], im[3][3];
+    auto rows = [&] {
 #pragma unroll
-    for (int a = 0; a < 3; ++a)
+        for (int a = 0; a < 3; ++a)
 #pragma unroll
-        for (int b = 0; b < 3; ++b) {
-            r[a][b] = w.r[3 * a + b];
-            im[a][b] = w.i[3 * a + b];
+            for (int b = 0; b < 3; ++b) {
+                r[a][b] = w.r[3 * a + b];
+                im[a][b] = w.i[3 * a + b];
+            }
+    };
+    rows();
+    if constexpr (sizeof(W) == 4) {
+        if (!fix_su3_rows_f32<SumFB>(r, im)) {  // far from SU(3): sums of any size
+            rows();
+            fix_su3_rows_f32<SumFF>(r, im);
         }
-    if constexpr (sizeof(W) == 4)
-        fix_su3_rows_f32(r, im);
-    else
+    } else {
         fix_su3_rows(r, im);
+    }
 #pragma unroll
     for (int a = 0; a < 3; ++a)
 #pragma unroll
@@ -370,7 +413,8 @@ __global__ void k_wflow_update(double2* links, Geom g, const double2* force, AHP
 // Bound by instruction issue (71%, three quarters of it FMA).  32^3x64, a step:
 // force and update apart 4.9 ms, fused 3.42 (128 registers; 168: 3.49, 96:
 // 3.48), with 32-bit offsets 3.22, with expm1_ah 3.03,
-// with the site coordinates by 32-bit divisions 2.94.
+// with the site coordinates by 32-bit divisions 2.94, with the shorter
+// compensated sums of FixSU3 (FB) 2.76.
 template <int STAGE, class L, typename I>
 __global__ void __launch_bounds__(128, 4)
     k_flow_stage32(L U, Geom g, AHPlanes<float> bbuf, float eps, float2* out) {

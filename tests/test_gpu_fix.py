@@ -15,7 +15,7 @@ import pytest
 torch = pytest.importorskip("torch")
 
 import oracle
-from flue_gb300 import _lib, generate
+from flue_gb300 import _lib, flow, generate
 from flue_gb300.field import as_field
 
 pytestmark = pytest.mark.gpu
@@ -245,3 +245,28 @@ def test_ensemble_mixes_fixed_point_and_fp64_fields():
             assert abs(r[2] - re) <= 1e-13 * v and abs(r[3] - im) <= 1e-13 * v
             b2 = G.magnetic(f)
             assert abs(r[4] - b2) <= 1e-14 * abs(b2) + 1e-28
+
+
+def _fix_su3_64(u):
+    """FixSU3Matrix of every link in complex128; u: (..., 3, 3)."""
+    r0 = u[..., 0, :] / np.linalg.norm(u[..., 0, :], axis=-1, keepdims=True)
+    r1 = u[..., 1, :] - r0 * np.sum(r0.conj() * u[..., 1, :], axis=-1, keepdims=True)
+    r1 = r1 / np.linalg.norm(r1, axis=-1, keepdims=True)
+    return np.stack([r0, r1, np.cross(r0, r1).conj()], axis=-2)
+
+
+# Rows of length^2 within 1/2 of 1 take sums of bounded size, others sums of any
+# size: both sides of the two limits, and rows of different length.  The step is
+# so short that it only reunitarises, three times.  Of an entry below 1 each time
+# rounds at most 2^-24, the entries of row 2 once more by the errors of rows 0
+# and 1 (two vectors of six such errors, 5 2^-24): 16 2^-24 in all.
+@pytest.mark.parametrize("rows", [(1.0, 1.0), (1.22, 1.0), (1.23, 1.0), (0.71, 1.0), (0.70, 1.0), (1.0, 1.22), (1.0, 1.23),
+                                  (1.0, 0.71), (1.0, 0.70), (3.0, 0.2)])
+def test_fp32_flow_reunitarises(rows):
+    u = generate.random_field((5, 3, 2, 3), 0.4, 11)
+    v = (u * np.array([rows[0], rows[1], 1.0])[:, None]).astype(np.complex64)
+    f = as_field(v, "c64")
+    ref = _fix_su3_64(v.astype(np.complex128))
+    flow.wflow_step(f, 1e-30)
+    got = f.to_numpy()
+    assert np.abs(got.astype(np.complex128) - ref).max() <= 16 * 2.0**-24

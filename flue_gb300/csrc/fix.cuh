@@ -584,42 +584,6 @@ __device__ __forceinline__ FxR ah_row(const Fx v[9], int a) {
     fx_row_sums<false>(m);
     return m;
 }
-// K^2 of an anti-Hermitian K (|K| <= 1): Hermitian, as its real diagonal and
-// upper triangle in the same order
-__device__ __forceinline__ void fx_ah_square(const Fx v[9], Fx y[9]) {
-    const Fx &br = v[3], &bi = v[4], &cr = v[5], &ci = v[6], &er = v[7], &ei = v[8];
-    auto sum = [](auto... t) {
-        FxAcc s = {FX_HI0, FX_CR0};
-        auto add = [&](const Fx& p, const Fx& q) { fx_mad(s, p, q); };
-        (t(add), ...);
-        return fx_limbs(s);
-    };
-    auto neg2 = [](const Fx& p) { return [p](auto add) { add(fx_neg(p), p); }; };        // - p^2
-    auto mul = [](const Fx& p, const Fx& q) { return [p, q](auto add) { add(p, q); }; };  // p q
-    y[0] = sum(neg2(v[0]), neg2(br), neg2(bi), neg2(cr), neg2(ci));
-    y[1] = sum(neg2(v[1]), neg2(br), neg2(bi), neg2(er), neg2(ei));
-    y[2] = sum(neg2(v[2]), neg2(cr), neg2(ci), neg2(er), neg2(ei));
-    // i (K00 + K11) b - c e*, i (K00 + K22) c + b e, i (K11 + K22) e - b* c
-    const Fx s01 = fx_add(v[0], v[1]), s02 = fx_add(v[0], v[2]), s12 = fx_add(v[1], v[2]);
-    y[3] = sum(mul(fx_neg(bi), s01), mul(fx_neg(cr), er), mul(fx_neg(ci), ei));
-    y[4] = sum(mul(br, s01), mul(fx_neg(ci), er), mul(cr, ei));
-    y[5] = sum(mul(fx_neg(ci), s02), mul(br, er), mul(fx_neg(bi), ei));
-    y[6] = sum(mul(cr, s02), mul(br, ei), mul(bi, er));
-    y[7] = sum(mul(fx_neg(ei), s12), mul(fx_neg(br), cr), mul(fx_neg(bi), ci));
-    y[8] = sum(mul(er, s12), mul(fx_neg(br), ci), mul(bi, cr));
-}
-// row a of that Hermitian matrix
-__device__ __forceinline__ FxR he_row(const Fx v[9], int a) {
-    FxR m;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        const Fx im = (a + c) == 1 ? v[4] : (a + c) == 2 ? v[6] : v[8];
-        m.r[c] = (a == c) ? v[a] : (a + c) == 1 ? v[3] : (a + c) == 2 ? v[5] : v[7];
-        m.i[c] = (a == c) ? Fx{0, 0} : a < c ? im : fx_neg(im);
-    }
-    fx_row_sums<false>(m);
-    return m;
-}
 // column b (the same in a whole warp) of K
 __device__ __forceinline__ FxV ah_col(const Fx v[9], int b) {
     FxV x;

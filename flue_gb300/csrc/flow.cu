@@ -459,8 +459,10 @@ __global__ void __launch_bounds__(128, 4)
 // moves it in one kernel from one fixed-point field to the other, and the last
 // stage writes the complex128 links.  A thread carries one column of a link
 // (three warps for 32 sites), as the 5-loop kernels do.  A stage is 13 matrix
-// products and the Taylor terms of exp(X) a link, bound by the integer
-// multiply-add pipe; 24^3x48: 13.5 ms as FP64 force and update, 2.4 ms so.
+// products and exp(X) a link, bound by the integer multiply-add pipe.  RK3 step
+// at 32^3x64: 92.8 ms as FP64 force and update, 22.2 with exp(X) from its even
+// and odd powers on the column, 21.0 with the weights of I, X and X^2 (a third
+// of the exponential's products).
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(128) k_flow_links(FullLinks<double> U, Geom g, MatFix w, FixGate gt) {
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -586,48 +588,84 @@ __global__ void __launch_bounds__(3 * FF_BS)
 #pragma unroll
         for (int e = 0; e < 9; ++e) x[e] = fx_of61((((i64)x[e].h << 32) + 2 * (i64)x[e].l) >> 1);
     }
-    // exp(X) U - U = [sum Y^j / (2j)!] U + X [sum Y^j / (2j+1)!] U, Y = X^2
-    // Hermitian: half the matrix-vector products of the plain series
-    Fx y[9];
-    fx_ah_square(x, y);
+    // exp(X) U - U = w0 U + w1 X U + w2 X (X U), the weights from the recurrence
+    // of X^k = p + q X + r X^2 with X^3 = -m X + i delta (expm1_ah; X has no trace).
+    // At even k p and r are real and q imaginary, at odd k the other way round,
+    // so an order takes two real products, and three into the weights.
+    FxR w3;
+    {
+        const Fx d0 = x[0], d1 = x[1], d2 = x[2], br = x[3], bi = x[4], cr = x[5], ci = x[6], er = x[7], ei = x[8];
+        auto sum2 = [](const Fx& a, const Fx& b, const Fx& c, const Fx& d) {  // a b + c d
+            FxAcc t = {FX_HI0, FX_CR0};
+            fx_mad(t, a, b), fx_mad(t, c, d);
+            return fx_limbs(t);
+        };
+        const Fx bb = sum2(br, br, bi, bi), cc = sum2(cr, cr, ci, ci), ee = sum2(er, er, ei, ei);
+        const Fx ber = sum2(br, er, fx_neg(bi), ei), bei = sum2(br, ei, bi, er);
+        FxAcc t = {0, FX_CR0};
+        fx_mad(t, d0, d0), fx_mad(t, d1, d1), fx_mad(t, d2, d2);
+        // -m = -|X|^2 / 2
+        const Fx nm = fx_of58(-((fx_fold(t) >> 1) + ((fx_int60(bb) + fx_int60(cc) + fx_int60(ee)) >> 2)));
+        t = {FX_HI0, FX_CR0};
+        fx_mad(t, fx_neg(d0), d1);
+        const Fx dd = fx_limbs(t);
+        FxAcc u2 = {0, FX_CR0};
+        fx_mad(u2, ber, ci), fx_mad(u2, fx_neg(bei), cr);
+        t = {FX_HI0 + 2 * fx_fold(u2), FX_CR0};
+        fx_mad(t, d1, cc), fx_mad(t, d2, bb), fx_mad(t, d0, ee), fx_mad(t, dd, d2);
+        const Fx delta = fx_limbs(t), ndelta = fx_neg(delta);
+        FxAcc wr[3], wi[3];
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+            wr[e] = {FX_HI0 + (e ? (i64)1 << (59 - e) : 0), FX_CR0};
+            wi[e] = {FX_HI0, FX_CR0};
+        }
+        // from X^2: p = q = 0, r = 1
+        Fx p = {0, 0}, q = {0, 0}, r = {1 << 29, 0};
+        float bnd = 0.5f * nrm * nrm;
+        auto next = [&](int k, const Fx& dl, FxAcc& a0, FxAcc& a1, FxAcc& a2) {
+            FxAcc tp = {FX_HI0, FX_CR0};
+            fx_mad(tp, dl, r);
+            FxAcc tq = {FX_HI0 + ((i64)p.h << 29), FX_CR0 + ((i64)p.l << 29)};
+            fx_mad(tq, nm, r);
+            r = q;
+            p = fx_limbs(tp);
+            q = fx_limbs(tq);
+            const Fx f = c_flow_fact.f[k];
+            fx_mad(a0, p, f), fx_mad(a1, q, f), fx_mad(a2, r, f);
+        };
+#pragma unroll 1
+        for (int k = 3; k < FLOW_TERMS; k += 2) {
+            bnd *= nrm / (float)k;  // |X|^k / k!
+            if (!(bnd > 0x1p-60f)) break;
+            next(k, delta, wi[0], wr[1], wi[2]);
+            next(k + 1, ndelta, wr[0], wi[1], wr[2]);
+            bnd *= nrm / (float)(k + 1);
+        }
+#pragma unroll
+        for (int e = 0; e < 3; ++e) w3.r[e] = fx_limbs(wr[e]), w3.i[e] = fx_limbs(wi[e]);
+        fx_row_sums<false>(w3);
+    }
     FxV u = w.col<false>(s, mu, b);
 #pragma unroll 1
     for (int rep = 0; rep < reps; ++rep) {
-        FxAcc er[3], ei[3], odr[3], odi[3];
+        FxV v, z;
+        FxVP vp = fx_prep<false>(u);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) fx_rdot_limbs(v.r[a], v.i[a], ah_row(x, a), vp);
+        vp = fx_prep<false>(v);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) fx_rdot_limbs(z.r[a], z.i[a], ah_row(x, a), vp);
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            er[a] = ei[a] = {0, FX_CR0};
-            odr[a] = odi[a] = {FX_HI0, FX_CR0};
-            fx_mad(odr[a], u.r[a], c_flow_fact.f[1]), fx_mad(odi[a], u.i[a], c_flow_fact.f[1]);
-        }
-        FxV t = u;
-        float bnd = nrm;
-#pragma unroll 1
-        for (int k = 2; k < FLOW_TERMS; k += 2) {
-            bnd *= nrm / (float)k;  // |X|^k / k!
-            if (!(bnd > 0x1p-60f)) break;
-            const FxVP tp = fx_prep<false>(t);
-#pragma unroll
-            for (int a = 0; a < 3; ++a) fx_rdot_limbs(t.r[a], t.i[a], he_row(y, a), tp);
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                fx_mad(er[a], t.r[a], c_flow_fact.f[k]), fx_mad(ei[a], t.i[a], c_flow_fact.f[k]);
-                fx_mad(odr[a], t.r[a], c_flow_fact.f[k + 1]), fx_mad(odi[a], t.i[a], c_flow_fact.f[k + 1]);
-            }
-            bnd *= nrm / (float)(k + 1);
-        }
-        FxVS d;
-        FxV o;
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            d.r[a] = fx_fold(er[a]), d.i[a] = fx_fold(ei[a]);
-            o.r[a] = fx_limbs(odr[a]), o.i[a] = fx_limbs(odi[a]);
-        }
-        fx_add_kv(d, x, fx_prep<false>(o));
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            u.r[a] = fx_const60(fx_int60(u.r[a]) + 4 * d.r[a]);
-            u.i[a] = fx_const60(fx_int60(u.i[a]) + 4 * d.i[a]);
+            FxV o;
+            o.r[0] = u.r[a], o.i[0] = u.i[a];
+            o.r[1] = v.r[a], o.i[1] = v.i[a];
+            o.r[2] = z.r[a], o.i[2] = z.i[a];
+            FxAcc dr, di;
+            fx_rdot(dr, di, w3, fx_prep<false>(o), 0, 0);
+            u.r[a] = fx_const60(fx_int60(u.r[a]) + 4 * fx_fold(dr));
+            u.i[a] = fx_const60(fx_int60(u.i[a]) + 4 * fx_fold(di));
         }
     }
     if (!live) return;

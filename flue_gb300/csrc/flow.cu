@@ -502,10 +502,14 @@ static __constant__ FlowFact c_flow_fact = flow_fact();
 struct FlowStage {
     Fx off, diag, last;
 };
-constexpr int FF_BS = 128;  // sites a block
+// Sites a block: the three columns meet at one barrier, so many small blocks
+// wait less for it than one large one.  RK3 step at 32^3x64: 128 sites 21.0 ms,
+// 64 with two / three blocks an SM 18.5 / 17.7, 32 with four / five / six / seven
+// 17.6 / 17.2 / 17.2 / 17.5.
+constexpr int FF_BS = 32, FF_MINB = 5;
 
 template <int STAGE, typename I>
-__global__ void __launch_bounds__(3 * FF_BS)
+__global__ void __launch_bounds__(3 * FF_BS, FF_MINB)
     k_flow_stage(Geom g, MatFix w, MatFix wout, AHFix xb, FlowStage sc, double2* links, FixGate gt) {
     __shared__ longlong2 sq[9][FF_BS];
     if (!gt.open()) return;

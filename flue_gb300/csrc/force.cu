@@ -193,19 +193,21 @@ struct MinBlocks<float> {
 };
 constexpr int FWD_BS = FLUE_FWD_BS;
 // Sites a block of the fixed-point forward and line cotangents covers, three
-// threads a site: 384 threads and up to 168 registers, one block an SM.  Both
+// threads a site: 192 threads and up to 168 registers, two blocks an SM.  Both
 // are bound by the integer multiply-add pipe (73% busy, waits on its results
-// next), so registers count for more than warps: B^2 force at 32^3x64 63.0 ms;
-// 64 sites with two blocks an SM 63.2, three (112 registers, spills) 67.6; 32
-// sites with four or five blocks 69.2, 69.9.
-constexpr int FIX_BS = 128;
-// The forward of a small lattice takes blocks of 32 sites, four an SM: below
-// three blocks of 128 sites an SM the last wave is mostly empty.  B^2 at 8^3x16
-// 194 -> 173 us, 10^3x16 254 -> 241, 12^3x24 497 -> 511 (so not there); two
-// halves of the leaves on twice the threads gave 182, 272, 502.
+// next), so registers count for more than warps.  32^3x64 in one pass, forward /
+// line cotangents: 128 sites (one block: its last warps leave an SM idle) 18.9 /
+// 43.8 ms, 64 18.5 / 42.3, 32 21.8 / 43.6; three blocks of 64 (112 registers)
+// spill.  In time slabs on four streams B^2 19.4 -> 19.0 ms.
+constexpr int FIX_BS = 64;
+// The forward of a small lattice takes blocks of 32 sites, four an SM: with few
+// blocks the last wave is mostly empty.  B^2 at 8^3x16 194 -> 173 us against 128
+// sites, 10^3x16 254 -> 241, 12^3x24 497 -> 511 (so not there: the line lies at
+// 3 x 128 sites and planes an SM); two halves of the leaves on twice the threads
+// gave 182, 272, 502.
 constexpr int FIX_BS_SMALL = 32;
 static int fix_fwd_block(int64_t V, int planes) {
-    return (V + FIX_BS - 1) / FIX_BS * planes < 3 * device_sms() ? FIX_BS_SMALL : FIX_BS;
+    return (V + 127) / 128 * planes < 3 * device_sms() ? FIX_BS_SMALL : FIX_BS;
 }
 
 // site j of the bs sites of block b of the forward's grid, plane p = b % np
@@ -258,9 +260,9 @@ __global__ void __launch_bounds__(FWD_BS)
 // Forward in fixed point: the sites and partial sums of the FP64 blocks, three
 // warps (columns) for every 32 sites.  32^3x64, three planes: FP64 pipe 81.1 ms,
 // fixed point with a thread a site 20.7 ms (240 registers, 8 warps an SM), with
-// a thread a column 19.0 ms.
+// a thread a column 18.5 ms.
 template <int BS, typename I>
-__global__ void __launch_bounds__(3 * BS, FIX_BS / BS)
+__global__ void __launch_bounds__(3 * BS, 128 / BS)
     k_fwd_fix(Geom g, PlaneArg pa, int kind, PatchArg pt, MatFix lines, AHFix kout, RefOut<double> fout, double* part,
               u32* kmax, bool kslice, FixGate gt) {
     __shared__ longlong2 sq[9][BS];
@@ -590,9 +592,9 @@ __global__ void __launch_bounds__(COT_BS) k_linecot_gated(Geom g, PlaneArg pa, M
 // line cotangents in fixed point: Lambda (180/512)^2 2^ks / 8, three warps
 // (columns) for every 32 sites.  X K(P) mixes the columns of X, which the three
 // warps exchange once a plane.  32^3x64: FP64 pipe 202 ms; a thread a site
-// 51.8 ms (its 255 registers spill), a thread a column 42.0 ms.
+// 51.8 ms (its 255 registers spill), a thread a column 42.3 ms.
 template <typename I>
-__global__ void __launch_bounds__(3 * FIX_BS)
+__global__ void __launch_bounds__(3 * FIX_BS, 128 / FIX_BS)
     k_linecot_fix(Geom g, PlaneArg pa, MatFix lines, AHFix kin, MatFix lam, const u32* kmax, bool kslice, FixGate gt) {
     __shared__ int4 sx[9][FIX_BS];
     if (!gt.open()) return;

@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(BS, (FlowMinBlocks<T, BS>::value)) k_ens_flow(
 constexpr int EF_BS = 128;
 template <int CH>
 __global__ void __launch_bounds__(3 * EF_BS) k_ens_flow_fix(EnsFlowArgs a) {
-    __shared__ longlong2 sq[9][EF_BS];
+    __shared__ longlong2 sq2[2][9][EF_BS];  // in turn: one barrier a plane
     __shared__ double sh[32];
     __shared__ int cur, ok;
     int* const err = a.ctr + 1;
@@ -389,11 +389,14 @@ __global__ void __launch_bounds__(3 * EF_BS) k_ens_flow_fix(EnsFlowArgs a) {
                 if (threadIdx.x == 0) ok = flow_wait(lines_done + j, sl.nchunk, err);
                 __syncthreads();
                 double e = 0.0;
+                int par = 0;
 #pragma unroll 1
                 for (int h = 0; h < CH && ok; h += EF_BS) {
                     const int64_t s = (int64_t)tk.b * CH + h + jt;
 #pragma unroll 1
                     for (int p = 0; p < a.pa.np; ++p) {
+                        longlong2(*sq)[EF_BS] = sq2[par];
+                        par ^= 1;
                         if (s < g.V) {
                             int c[4];
                             site_coords(g, s, c);
@@ -409,7 +412,6 @@ __global__ void __launch_bounds__(3 * EF_BS) k_ens_flow_fix(EnsFlowArgs a) {
                             fx_field_strength(d, FXQ5, fv);
                             e += ah_norm2(fv);
                         }
-                        __syncthreads();
                     }
                 }
                 const double r = block_sum(e, sh);

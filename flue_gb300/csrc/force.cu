@@ -591,12 +591,13 @@ __global__ void __launch_bounds__(COT_BS) k_linecot_gated(Geom g, PlaneArg pa, M
 
 // line cotangents in fixed point: Lambda (180/512)^2 2^ks / 8, three warps
 // (columns) for every 32 sites.  X K(P) mixes the columns of X, which the three
-// warps exchange once a plane.  32^3x64: FP64 pipe 202 ms; a thread a site
-// 51.8 ms (its 255 registers spill), a thread a column 42.3 ms.
+// warps exchange once a plane, through two buffers in turn (one barrier a plane:
+// 42.3 -> 41.3 ms; barriers of the three warps alone 41.5).  32^3x64: FP64 pipe 202 ms; a thread a site
+// 51.8 ms (its 255 registers spill), a thread a column 41.3 ms.
 template <typename I>
 __global__ void __launch_bounds__(3 * FIX_BS, 128 / FIX_BS)
     k_linecot_fix(Geom g, PlaneArg pa, MatFix lines, AHFix kin, MatFix lam, const u32* kmax, bool kslice, FixGate gt) {
-    __shared__ int4 sx[9][FIX_BS];
+    __shared__ int4 sx2[2][9][FIX_BS];
     if (!gt.open()) return;
     const int ntask = 3 * pa.nd;
     const int task = blockIdx.x % ntask;
@@ -619,6 +620,7 @@ __global__ void __launch_bounds__(3 * FIX_BS, 128 / FIX_BS)
     const int nw = len == 1 ? 3 : 2;
     const int ks = kscale(kmax + (kslice ? c[0] : 0));
     FxVS acc = vs_zero();
+    int par = 0;
 #pragma unroll 1
     for (int p = 0; p < pa.np; ++p) {
         const int pmu = sel(pa.mu, p), pnu = sel(pa.nu, p);
@@ -640,6 +642,8 @@ __global__ void __launch_bounds__(3 * FIX_BS, 128 / FIX_BS)
             line_side_fix<-1>(acc, X, cw, lines, kin, p, ks, s, Q, (I)((int64_t)wrapd(cf, -w, nf) * stf), pf, pB, b);
         }
         const FxV x = fx_of58(X);
+        int4(*sx)[FIX_BS] = sx2[par];
+        par ^= 1;
 #pragma unroll
         for (int a = 0; a < 3; ++a) sx[3 * a + b][jt] = make_int4(x.r[a].h, x.r[a].l, x.i[a].h, x.i[a].l);
         Fx kv[9];
@@ -660,7 +664,6 @@ __global__ void __launch_bounds__(3 * FIX_BS, 128 / FIX_BS)
             fx_row_sums<false>(m);
             fx_rdot_add(acc, a, m, kc);
         }
-        __syncthreads();
     }
     if (live) {
 #pragma unroll

@@ -553,6 +553,9 @@ __global__ void __launch_bounds__(3 * FF_BS, FF_MINB)
 #pragma unroll
         for (int a = 0; a < 3; ++a) sq[3 * a + b][j] = make_longlong2(un.r[a], un.i[a]);
     }
+    // X_last before the barrier: the first column's warp overwrites it after
+    Fx last[9];
+    if (STAGE > 0) xb.load(s, mu, 0, last);
     __syncthreads();
     // X = sc . (U N - (U N)^+ without its trace) + sc.last X_last
     Fx x[9];
@@ -561,8 +564,6 @@ __global__ void __launch_bounds__(3 * FF_BS, FF_MINB)
         fx_antiherm([&](int el) { return sq[el][j]; }, d);
         // (diagonal entries of fx_antiherm are 2 Im: 3 Im - trace from them)
         const i64 tr = (d[0] + d[1] + d[2]) >> 1;
-        Fx last[9];
-        if (STAGE > 0) xb.load(s, mu, 0, last);
 #pragma unroll
         for (int e = 0; e < 9; ++e) {
             const i64 de = e < 3 ? d[e] + (d[e] >> 1) - tr : d[e];
@@ -577,7 +578,7 @@ __global__ void __launch_bounds__(3 * FF_BS, FF_MINB)
             xb.store(s64, mu, d);
         }
     }
-    // exp(X) U by Taylor on the column, X halved until |X|_F <= 1/2
+    // X halved until |X|_F <= 1/2
     float nrm = 0.f;
 #pragma unroll
     for (int e = 0; e < 9; ++e) {

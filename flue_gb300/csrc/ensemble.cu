@@ -12,7 +12,11 @@
 //   COLS(f, c):  spatial and temporal plaquettes and the Polyakov loops of a
 //                run of time columns of field f.
 // FWD(j, .) waits until every LINES(j, .) has finished, and LINES(j, .)
-// waits until every FWD(j - kSlots, .) has released the slot.  The list
+// waits until every FWD(j - kSlots, .) has released the slot.  complex128
+// fields are shared out between two launches, fixed point and FP64, one after
+// the other: each skips the tasks of the other's fields, and its LINES(j, .)
+// wait for the last slab of the slot that it did not skip (ring_prev; a skipped
+// slab says nothing of the one before it).  The list
 // places LINES(j) before FWD(j - 1), so every task waits only on tasks with
 // lower indices: those were taken by resident blocks and finish, so the
 // schedule always progresses.  Every wait is bounded; a wait that runs out
@@ -99,6 +103,19 @@ __device__ __forceinline__ bool ens_any(const EnsFlowArgs& a, bool open) {
     bool any = false;
     for (int f = threadIdx.x; f < a.nfields; f += blockDim.x) any = any || ens_open(a, f) == open;
     return __syncthreads_or(any);
+}
+
+// The slab whose FWD tasks have to be done before this launch writes the lines
+// of slab j: the last one of j's ring slot among the fields it takes, those whose
+// gate is `open` (-1: none).  Called by a whole warp; a turn looks at 32 slabs.
+__device__ __forceinline__ int ring_prev(const EnsFlowArgs& a, int j, bool open, bool mixed) {
+    if (!mixed) return j < kSlots ? -1 : j - kSlots;
+    for (int i0 = j - kSlots; i0 >= 0; i0 -= 32 * kSlots) {
+        const int i = i0 - kSlots * (int)(threadIdx.x & 31);
+        const u32 own = __ballot_sync(0xffffffffu, i >= 0 && ens_open(a, a.slabs[max(i, 0)].field) == open);
+        if (own) return i0 - kSlots * (__ffs((int)own) - 1);
+    }
+    return -1;
 }
 
 // Counts every field's links in its gate (all four directions: a quarter of
@@ -195,6 +212,7 @@ __global__ void __launch_bounds__(BS, (FlowMinBlocks<T, BS>::value)) k_ens_flow(
     int* const fwd_done = a.ctr + 2 + a.nslabs;
     // complex128: only the fields that the fixed-point kernel left out
     if (a.gates && !ens_any(a, false)) return;
+    const bool mixed = a.gates && ens_any(a, true);
     // every task is taken once: at most ntasks + 1 turns per block
     for (int guard = 0; guard <= a.ntasks; ++guard) {
         if (threadIdx.x == 0) cur = atomicAdd(a.ctr, 1);
@@ -241,9 +259,11 @@ __global__ void __launch_bounds__(BS, (FlowMinBlocks<T, BS>::value)) k_ens_flow(
             const MatAoS<T> lines{reinterpret_cast<VP>(a.ring + (size_t)(j % kSlots) * a.slot_bytes), g.V};
             const int64_t s = (int64_t)tk.b * BS + threadIdx.x;
             if (tk.type == TASK_LINES) {
-                // the slot is free once every FWD task of slab j - kSlots is done
-                if (threadIdx.x == 0)
-                    ok = j < kSlots || flow_wait(fwd_done + (j - kSlots), a.slabs[j - kSlots].nchunk, err);
+                // the slot is free once every FWD task of its last slab is done
+                if (threadIdx.x < 32) {
+                    const int i = ring_prev(a, j, false, mixed);
+                    if (threadIdx.x == 0) ok = i < 0 || flow_wait(fwd_done + i, a.slabs[i].nchunk, err);
+                }
                 __syncthreads();
                 if (ok && s < g.V) {
                     const L U = LinksFrom<L>::make(f.links, f.g.V);
@@ -293,6 +313,7 @@ __global__ void __launch_bounds__(3 * EF_BS) k_ens_flow_fix(EnsFlowArgs a) {
     int* const fwd_done = a.ctr + 2 + a.nslabs;
     const int b = threadIdx.x / EF_BS, jt = threadIdx.x % EF_BS;
     if (!ens_any(a, true)) return;
+    const bool mixed = ens_any(a, false);
     for (int guard = 0; guard <= a.ntasks; ++guard) {
         if (threadIdx.x == 0) cur = atomicAdd(a.ctr, 1);
         __syncthreads();
@@ -372,8 +393,10 @@ __global__ void __launch_bounds__(3 * EF_BS) k_ens_flow_fix(EnsFlowArgs a) {
             const Geom g = make_geom(sl.nts, f.g.n[1], f.g.n[2], f.g.n[3]);
             const MatFix lines{(int4*)(a.ring + (size_t)(j % kSlots) * a.slot_bytes), g.V};
             if (tk.type == TASK_LINES) {
-                if (threadIdx.x == 0)
-                    ok = j < kSlots || flow_wait(fwd_done + (j - kSlots), a.slabs[j - kSlots].nchunk, err);
+                if (threadIdx.x < 32) {
+                    const int i = ring_prev(a, j, true, mixed);
+                    if (threadIdx.x == 0) ok = i < 0 || flow_wait(fwd_done + i, a.slabs[i].nchunk, err);
+                }
                 __syncthreads();
 #pragma unroll 1
                 for (int h = 0; h < CH && ok; h += EF_BS) {  // a thread a (site, direction)

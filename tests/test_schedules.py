@@ -126,3 +126,84 @@ def test_flow_stage_in_any_order_of_its_warps(tmp_path):
     exe = _build(tmp_path, body + FLOW_MAIN)
     r = subprocess.run([exe], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+ENS_MAIN = LINKS + r"""
+// Five fields of 18-site time slices, one slab a slice, every other one left to
+// the other scheduler; `part` after one scheduler over all of them.  turns: one resident
+// block each, and the waits it may take before the next one runs.
+static std::vector<double> run(const std::vector<int>& turns, bool fixed, std::vector<EnsTask>& tasks) {
+    const int nts[5] = {6, 5, 7, 6, 6};
+    std::vector<EnsField> fields;
+    std::vector<EnsSlab> slabs;
+    std::vector<std::vector<double2>> links(5);
+    std::vector<u32> gates;
+    Rng rng{7};
+    for (int f = 0; f < 5; ++f) {
+        const Geom g = make_geom(nts[f], 2, 3, 3);
+        links[f].resize(36 * g.V);
+        for (int mu = 0; mu < 4; ++mu)
+            for (int64_t s = 0; s < g.V; ++s) {
+                double r[3][3], i[3][3];
+                random_link(rng, r, i);
+                for (int a = 0; a < 3; ++a)
+                    for (int b = 0; b < 3; ++b) links[f][s + g.V * (mu + 4 * (a + 3 * b))] = {r[a][b], i[a][b]};
+            }
+        fields.push_back({links[f].data(), g});
+        for (int t = 0; t < nts[f]; ++t) slabs.push_back({f, t, 1, 1});
+        // fields 0, 2 and 4 are the scheduler's own (FP64: those that are shut)
+        gates.push_back((f % 2 == 0) != fixed), gates.push_back((u32)(4 * g.V));
+    }
+    const int ns = (int)slabs.size();
+    tasks.clear();
+    for (int j = 0; j <= ns; ++j) {
+        if (j < ns) tasks.push_back({TASK_LINES, j, 0, 0});
+        if (j >= 1) tasks.push_back({TASK_FWD, j - 1, 0, 0});
+    }
+    const size_t slot = std::max(MatFix::bytes(18, 9), MatAoS<double>::bytes(18, 9));
+    std::vector<int> ctr(2 + 2 * ns);
+    std::vector<double> part(tasks.size() * NOBS);
+    std::vector<longlong2> ring(kSlots * slot / 16);
+    EnsFlowArgs a{};
+    a.fields = fields.data(), a.slabs = slabs.data(), a.tasks = tasks.data();
+    a.ntasks = (int)tasks.size(), a.nslabs = ns, a.ctr = ctr.data(), a.part = part.data();
+    a.ring = (char*)ring.data(), a.slot_bytes = slot, a.nfields = 5, a.gates = gates.data();
+    const int mu[3] = {2, 1, 3}, nu[3] = {1, 3, 2}, sl[4] = {-1, 1, 0, 2}, dir[3] = {2, 1, 3};
+    a.pa.np = 3, a.pa.nd = 3;
+    for (int k = 0; k < 4; ++k) a.pa.slot[k] = sl[k], a.pa.dir[k] = k < 3 ? dir[k] : -1;
+    for (int k = 0; k < 3; ++k) a.pa.mu[k] = mu[k], a.pa.nu[k] = nu[k];
+    if (fixed)
+        emu::launch_resident(3 * EF_BS, turns, [&] { k_ens_flow_fix<128>(a); });
+    else
+        emu::launch_resident(128, turns, [&] { k_ens_flow<FullLinks<double>, double, 128>(a); });
+    if (ctr[1]) part.assign(part.size(), -1.0);  // a wait ran out
+    return part;
+}
+}  // namespace flue
+int main() {
+    using namespace flue;
+    std::vector<EnsTask> tasks;
+    for (bool fixed : {true, false}) {
+        const auto want = run({1}, fixed, tasks);
+        std::vector<std::vector<int>> speeds{{1, 1}, {1, 30, 30}, {30, 1, 5}};
+        for (int n = 40; n <= 400; n += 30) speeds.push_back({1, n}), speeds.push_back({n, 2, n});
+        for (const std::vector<int>& turns : speeds) {
+            const auto got = run(turns, fixed, tasks);
+            for (size_t t = 0; t < tasks.size(); ++t)
+                if (tasks[t].type == TASK_FWD && got[t * NOBS + 4] != want[t * NOBS + 4])
+                    return printf("%s: slab %d, %zu blocks\n", fixed ? "fixed point" : "FP64", tasks[t].a, turns.size()), 1;
+        }
+    }
+    return 0;
+}
+"""
+
+
+def test_ensemble_ring_in_any_order_of_its_blocks(tmp_path):
+    """Fields that a scheduler owns between fields that it skips, blocks of very
+    different speed: no slab's lines are overwritten while they are read."""
+    ens = _source("ensemble.cu")
+    body = _cut(ens, "constexpr int NOBS = 6;\n", "// out[f*NOBS + o] = sum of the field's task partials")
+    exe = _build(tmp_path, body + ENS_MAIN)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stdout + r.stderr

@@ -468,10 +468,17 @@ __global__ void __launch_bounds__(128) k_flow_links(FullLinks<double> U, Geom g,
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     u32 st = 0;
     if (s < g.V) {
-        const M3<double> u = U.load(s, (int)blockIdx.y);
+        const int mu = (int)blockIdx.y;
+        const M3<double> u = U.load(s, mu);
         const M3F f = fx_of(u);
         st = link_state(u, f);
-        w.store(s, (int)blockIdx.y, f);
+        w.store(s, mu, f);
+        if (st == 0) {
+            int c[4];
+            site_coords(g, s, c);
+            for (int nu = mu + 1; nu < 4; ++nu)
+                if (near_patch(U, g, c, mu, nu)) st = 1;
+        }
     }
     gate_count(gt, st);
 }

@@ -139,13 +139,23 @@ __global__ void k_lines(L U, Geom g, Geom gs, int t0, PlaneArg pa, MatAoS<T> lin
 }
 
 // complex128 fields: the lines in fixed point (fix.cuh), counting the links
-// that are not unitary, or close to 1, in the gate.  32^3x64 B^2: 1.06 ms, HBM
+// that are not unitary, or close to 1 together, in the gate.  32^3x64 B^2: 1.06 ms, HBM
 // (2.7 GB written) and the conversion of the links to limbs.
 __global__ void __launch_bounds__(128) k_lines_fix(FullLinks<double> U, Geom g, Geom gs, int t0, PlaneArg pa,
                                                    MatFix lines, FixGate gt) {
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int slot = (int)blockIdx.y;
     u32 st = 0;
-    if (s < g.V) st = line_site_fix(U, g, gs, t0, pa, lines, s, (int)blockIdx.y);
+    if (s < g.V) {
+        st = line_site_fix(U, g, gs, t0, pa, lines, s, slot);
+        if (st == 0) {
+            int c[4];
+            site_coords(g, s, c);
+            c[0] += t0;
+            for (int k = slot + 1; k < pa.nd; ++k)
+                if (near_patch(U, gs, c, sel(pa.dir, slot), sel(pa.dir, k))) st = 1;
+        }
+    }
     gate_count(gt, st);
 }
 
@@ -250,11 +260,16 @@ __global__ void __launch_bounds__(FWD_BS, MinBlocks<T>::fwd)
 template <typename I>
 __global__ void __launch_bounds__(FWD_BS)
     k_fwd_gated(Geom g, PlaneArg pa, int kind, PatchArg pt, MatAoS<double> lines, AHAoS<double> kout,
-                RefOut<double> fout, double* part, unsigned nblocks, FixGate gt) {
+                RefOut<double> fout, double* part, unsigned nblocks, unsigned nparts, FixGate gt) {
     __shared__ double sh[32];
     if (gate_shut(gt)) return;
     for (unsigned b = blockIdx.x; b < nblocks; b += gridDim.x)
         fwd_block<double, I>(b, g, pa, kind, pt, lines, kout, fout, part, sh);
+    // the smaller blocks of the fixed-point forward have more partial sums: with
+    // zeros for the rest the energy is that of the ungated kernel, bit for bit
+    if (part)
+        for (unsigned b = nblocks + blockIdx.x * blockDim.x + threadIdx.x; b < nparts; b += gridDim.x * blockDim.x)
+            part[b] = 0.0;
 }
 
 // Forward in fixed point: the sites and partial sums of the FP64 blocks, three
@@ -976,11 +991,15 @@ static cudaError_t energy_fwd_part(const L& U, const Geom& g, const Geom& gs, in
             else
                 fwd(k_fwd_fix<FIX_BS, int64_t>);
         }
-        const unsigned nf = nbx * pa.np, gf = gated_grid(w, nf);
+        const unsigned nf = (unsigned)((g.V + FWD_BS - 1) / FWD_BS) * pa.np, gf = gated_grid(w, nf);
+        const PatchArg pt64 = FLUE_FWD_PATCH ? make_patch(g, pa, FWD_BS) : PatchArg{};
+        auto fwd64 = [&](auto kernel) {
+            note_launch(), kernel<<<gf, FWD_BS, 0, st>>>(g, pa, kind, pt64, lines, kb, fout, part, nf, nbx * pa.np, gt);
+        };
         if (fits)
-            note_launch(), k_fwd_gated<u32><<<gf, fbs, 0, st>>>(g, pa, kind, pt, lines, kb, fout, part, nf, gt);
+            fwd64(k_fwd_gated<u32>);
         else
-            note_launch(), k_fwd_gated<int64_t><<<gf, fbs, 0, st>>>(g, pa, kind, pt, lines, kb, fout, part, nf, gt);
+            fwd64(k_fwd_gated<int64_t>);
     } else {
         note_launch(), k_lines<L, T><<<dim3(nbl, pa.nd), 128, 0, st>>>(U, g, gs, t0, pa, lines);
         stage_mark(1, st);

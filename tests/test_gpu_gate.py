@@ -5,10 +5,11 @@ import pytest
 
 torch = pytest.importorskip("torch")
 
-from flue_gb300 import generate
+from flue_gb300 import _lib, generate
 from flue_gb300 import gluonCalc as G
 from flue_gb300.ensemble import Ensemble
 from flue_gb300.field import as_field
+from tests.test_gpu_fix import ALL, B2, _both, _flow_both
 
 pytestmark = pytest.mark.gpu
 
@@ -32,3 +33,39 @@ def test_ensemble_of_open_and_shut_fields_reuses_its_ring(block, monkeypatch):
     for f, r in zip(fields, first):
         b2 = G.magnetic(f)
         assert abs(r[4] - b2) <= 1e-14 * abs(b2)
+
+
+def _part_near_one(dims, dist, where):
+    """A Haar field with links near 1 in a part of it: half of the x extent, every
+    fourth time slice, or one direction at all sites."""
+    u, c = np.array(generate.haar_field(dims, 3)), np.array(generate.random_field(dims, dist, 4))
+    if where == "half":
+        u[:, dims[1] // 2:] = c[:, dims[1] // 2:]
+    elif where == "slices":
+        u[::4] = c[::4]
+    else:
+        u[..., 2, :, :] = c[..., 2, :, :]
+    return u
+
+
+# F, its gradient and the flow's X are small where all links are close to 1, and
+# FP64 has their error relative to that: such fields stay in FP64, bit for bit.
+@pytest.mark.parametrize("where", ["half", "slices"])
+@pytest.mark.parametrize("dist", [0.0, 1e-8, 1e-3, 0.01])
+def test_regions_near_one_stay_in_fp64(where, dist):
+    u = _part_near_one((8, 8, 4, 6), dist, where)
+    f = as_field(np.asfortranarray(u))
+    for planes in (B2, ALL, ((3, 4),)):
+        (e1, g1), (e0, g0) = _both(f, planes, _lib.FORCE_LIE)
+        assert e1 == e0 and np.array_equal(g1, g0)
+    a, b = _flow_both(u, 0.02)
+    assert np.array_equal(a, b)
+
+
+def test_one_direction_near_one_takes_fixed_point():
+    u = _part_near_one((8, 8, 4, 6), 1e-3, "direction")
+    (_, g1), (_, g0) = _both(as_field(np.asfortranarray(u)), B2, _lib.FORCE_LIE)
+    assert not np.array_equal(g1, g0)
+    assert np.linalg.norm(g1 - g0) <= 8e-15 * np.linalg.norm(g0)
+    a, b = _flow_both(u, 0.02)
+    assert not np.array_equal(a, b) and np.abs(a - b).max() <= 8 * 2.0**-53

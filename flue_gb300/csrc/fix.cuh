@@ -346,15 +346,14 @@ __device__ __forceinline__ i64 fx_rezdot(const FxV& u, const FxV& v) {
     for (int k = 0; k < 3; ++k) fx_mad(s, u.r[k], v.r[k]), fx_mad(s, u.i[k], v.i[k]);
     return fx_fold(s);
 }
-// Sum over a warp of integers |t| < 2^62 (exact, rounded once to the double):
-// three 22-bit parts by the warp's integer reduction, in place of five FP64
-// additions a lane.
-__device__ __forceinline__ double warp_sum_fix(i64 t) {
+// Sum over a warp of integers |t| < 2^60 of unit 2^-58, in units of 2^-54
+// (rounded once): three 22-bit parts by the warp's integer reduction.
+__device__ __forceinline__ i64 warp_sum_fix54(i64 t) {
     const u32 m = (1u << 22) - 1;
     const u32 s0 = __reduce_add_sync(0xffffffffu, (u32)t & m);
     const u32 s1 = __reduce_add_sync(0xffffffffu, (u32)(t >> 22) & m);
     const int s2 = __reduce_add_sync(0xffffffffu, (int)(t >> 44));
-    return fma((double)s2, 0x1p44, fma((double)s1, 0x1p22, (double)s0));
+    return ((i64)s2 << 40) + ((i64)s1 << 18) + ((s0 + 8) >> 4);
 }
 
 // ---------------------------------------------------------------------------

@@ -812,14 +812,15 @@ __global__ void __launch_bounds__(WT_BS) k_wt_lines_fix(FullLinks<double> U, Geo
 // part of the trace, two matrix-vector products a thread and loop.  32^3x64, 8 x
 // 8 table: FP64 58.8 ms; fixed point 22.6 ms with a barrier a loop, and with one
 // barrier 16.7 ms (128 sites a block, 12 warps an SM), 13.7 (64 sites, 18 warps,
-// 112 registers, spills), 13.4 (32 sites, 15 warps, 136 registers); 13.2 with the
-// site coordinates by 32-bit divisions.
+// 112 registers, spills), 13.4 (32 sites, 15 warps, 128 registers, 80-96 bytes of
+// stack); 13.2 with the site coordinates by 32-bit divisions, 12.3 with the sums
+// of a warp kept as integers (no conversion on the FP64 pipe).
 constexpr int WTF_BS = 32, WTF_WARPS = 3 * WTF_BS / 32, WT_MAXT = 64;
 
 template <typename I>
 __global__ void __launch_bounds__(3 * WTF_BS, 5)
-    k_wt_loops_fix(Geom g, int mu, int nu, int rmax, int tmax, MatFix lines, double* __restrict__ part, FixGate gt) {
-    __shared__ double sh[WT_MAXT][WTF_WARPS];  // one barrier for all the loops
+    k_wt_loops_fix(Geom g, int mu, int nu, int rmax, int tmax, MatFix lines, i64* __restrict__ part, FixGate gt) {
+    __shared__ i64 sh[WT_MAXT][WTF_WARPS];  // one barrier for all the loops
     if (!gt.open()) return;
     const int R = blockIdx.x % rmax + 1, sb = blockIdx.x / rmax, nsb = gridDim.x / rmax;
     const int b = threadIdx.x / WTF_BS, w = threadIdx.x >> 5;
@@ -840,15 +841,49 @@ __global__ void __launch_bounds__(3 * WTF_BS, 5)
         const I sT = (I)((int64_t)s + (ct - cn) * sn);
         const FxV ab = lines.mul<false>(s, R - 1, lines.col<false>(sR, rmax + T - 1, b));
         const FxV dc = lines.mul<false>(s, rmax + T - 1, lines.col<false>(sT, R - 1, b));
-        const double r = warp_sum_fix(live ? fx_rezdot(ab, dc) : 0);
+        const i64 r = warp_sum_fix54(live ? fx_rezdot(ab, dc) : 0);
         if ((threadIdx.x & 31) == 0) sh[T - 1][w] = r;
     }
     __syncthreads();
     if (threadIdx.x < tmax) {
-        double sum = 0.0;
+        i64 sum = 0;
 #pragma unroll
-        for (int k = 0; k < WTF_WARPS; ++k) sum += sh[threadIdx.x][k];
-        part[(int64_t)((R - 1) * tmax + threadIdx.x) * nsb + sb] = sum * 0x1p-58;
+        for (int k = 0; k < WTF_WARPS; ++k) sum += sh[threadIdx.x][k];  // at most 3 x 2^59
+        part[(int64_t)((R - 1) * tmax + threadIdx.x) * nsb + sb] = sum;
+    }
+}
+
+// Means of the loops from the block sums, a block a loop: integers of unit 2^-54,
+// added exactly (as FP64 sums the four times as many blocks of the fixed-point
+// kernel cost a tenth of an ulp at 32^3x64), or where the gate is shut the FP64
+// sums of n64 blocks as k_finish_sums takes them.
+__global__ void __launch_bounds__(256) k_wt_finish(const double* __restrict__ part, int nfix, int n64, double scale,
+                                                   FixGate gt, double* __restrict__ out) {
+    __shared__ double sh[32];
+    __shared__ i64 shl[8], shh[8];
+    if (!gt.open()) {
+        finish_sum(part + (int64_t)blockIdx.x * n64, n64, scale, out + blockIdx.x, sh);
+        return;
+    }
+    const i64* p = reinterpret_cast<const i64*>(part) + (int64_t)blockIdx.x * nfix;
+    i64 lo = 0, hi = 0;
+#pragma unroll 8
+    for (int i = threadIdx.x; i < nfix; i += 256) {
+        const i64 v = __ldcg(p + i);
+        lo += (u32)v;
+        hi += v >> 32;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        lo += __shfl_down_sync(0xffffffffu, lo, o);
+        hi += __shfl_down_sync(0xffffffffu, hi, o);
+    }
+    if ((threadIdx.x & 31) == 0) shl[threadIdx.x >> 5] = lo, shh[threadIdx.x >> 5] = hi;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < 8; ++k) lo += shl[k], hi += shh[k];
+        hi += lo >> 32;
+        out[blockIdx.x] = fma((double)hi, 0x1p-22, (double)(u32)lo * 0x1p-54) * scale;
     }
 }
 
@@ -890,15 +925,16 @@ cudaError_t launch_wmunu_table(const FieldRef& U, int mu, int nu, int rmax, int 
         const MatAoS<double> dl{(double2*)ws, g.V};
         const unsigned cap = 8u * (unsigned)device_sms(), nsf = (unsigned)((g.V + WTF_BS - 1) / WTF_BS);
         note_launch(), k_wt_lines_fix<<<dim3(nsb, 2), WT_BS, 0, st>>>(L, g, mu, nu, rmax, tmax, fl, gt);
+        i64* ipart = reinterpret_cast<i64*>(part);
         if (MatFix::fits32(g.V, rmax + tmax))
-            note_launch(), k_wt_loops_fix<u32><<<nsf * rmax, 3 * WTF_BS, 0, st>>>(g, mu, nu, rmax, tmax, fl, part, gt);
+            note_launch(), k_wt_loops_fix<u32><<<nsf * rmax, 3 * WTF_BS, 0, st>>>(g, mu, nu, rmax, tmax, fl, ipart, gt);
         else
-            note_launch(), k_wt_loops_fix<int64_t><<<nsf * rmax, 3 * WTF_BS, 0, st>>>(g, mu, nu, rmax, tmax, fl, part, gt);
+            note_launch(), k_wt_loops_fix<int64_t><<<nsf * rmax, 3 * WTF_BS, 0, st>>>(g, mu, nu, rmax, tmax, fl, ipart, gt);
         note_launch(), k_wt_lines_gated<<<std::min(nsb, cap), WT_BS, 0, st>>>(L, g, mu, nu, rmax, tmax, dl, gt);
-        note_launch(), k_wt_loops_gated<<<std::min(nsf * nrt, cap), WTF_BS, 0, st>>>(g, mu, nu, rmax, tmax, (int)nsf, dl,
-                                                                                    part, gt);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        return launch_finish_sums(part, (int)nsf, (int)nrt, out, st, 1.0 / (double)g.V);
+        note_launch(), k_wt_loops_gated<<<std::min(nsb * nrt, cap), WT_BS, 0, st>>>(g, mu, nu, rmax, tmax, (int)nsb, dl,
+                                                                                   part, gt);
+        note_launch(), k_wt_finish<<<nrt, 256, 0, st>>>(part, (int)nsf, (int)nsb, 1.0 / (double)g.V, gt, out);
+        return cudaGetLastError();
     }
     FLUE_DISPATCH_LINKS(U, {
         MatAoS<T> ln{reinterpret_cast<decltype(MatAoS<T>::p)>(ws), g.V};

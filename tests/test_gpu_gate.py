@@ -8,7 +8,7 @@ torch = pytest.importorskip("torch")
 from flue_gb300 import _lib, generate
 from flue_gb300 import gluonCalc as G
 from flue_gb300.ensemble import Ensemble
-from flue_gb300.field import as_field
+from flue_gb300.field import GaugeField, as_field
 from tests.test_gpu_fix import ALL, B2, _both, _flow_both
 
 pytestmark = pytest.mark.gpu
@@ -69,3 +69,17 @@ def test_one_direction_near_one_takes_fixed_point():
     assert np.linalg.norm(g1 - g0) <= 8e-15 * np.linalg.norm(g0)
     a, b = _flow_both(u, 0.02)
     assert not np.array_equal(a, b) and np.abs(a - b).max() <= 8 * 2.0**-53
+
+
+# The same links everywhere: every loop of a kind has one trace, and the mean over
+# 2^21 sites has to be that of 2^8 sites, in every bit.
+@pytest.mark.parametrize("seed", range(4))
+def test_wmunu_table_adds_its_loops_exactly(seed):
+    links = torch.as_tensor(np.array(generate.haar_field((1, 1, 1, 1), seed))[0, 0, 0, 0]).cuda()  # [mu, a, b]
+
+    def table(nt, n):
+        f = GaugeField.empty((nt, n, n, n), "c128")
+        f.storage.copy_(links.permute(2, 1, 0)[:, :, :, None, None, None, None].expand_as(f.storage))
+        return G.wmunu_table(f, 2, 1, 4, 4)
+
+    assert np.array_equal(table(64, 32), table(4, 4))

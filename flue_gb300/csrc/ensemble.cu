@@ -131,6 +131,7 @@ __global__ void __launch_bounds__(128) k_ens_gates(EnsFlowArgs a) {
         for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x; i0 < n; i0 += (int64_t)gridDim.x * blockDim.x) {
             const int64_t i = i0 + threadIdx.x;
             u32 st = 0;
+            if (gate_lost(gt)) break;
             if (i < n) {
                 const M3<double> u = U.load(i % fl.g.V, (int)(i / fl.g.V));
                 st = link_state(u, fx_of(u));

@@ -452,13 +452,21 @@ __device__ __forceinline__ bool near_patch(const FullLinks<double>& U, const Geo
 }
 
 // add one warp's link states to the gate (all 32 lanes call; st = 0 for idle
-// lanes); integer counts, so the result does not depend on the order
-__device__ __forceinline__ void gate_count(const FixGate& gt, u32 st) {
+// lanes); integer counts, so the result does not depend on the order.  Returns
+// the lanes of bit 0 and of bit 1.
+__device__ __forceinline__ uint2 gate_count(const FixGate& gt, u32 st) {
     const u32 bad = __ballot_sync(0xffffffffu, st & 1u), far = __ballot_sync(0xffffffffu, st & 2u);
     if ((threadIdx.x & 31) == 0) {
         if (bad) atomicAdd(gt.p, (u32)__popc(bad));
         if (far) atomicAdd(gt.p + 1, (u32)__popc(far));
     }
+    return make_uint2(bad, far);
+}
+
+// Whether a warp has met something that shuts the gate, whatever the others find:
+// what this one would still do is for nothing.  (The same answer in a whole warp.)
+__device__ __forceinline__ bool gate_lost(const FixGate& gt) {
+    return __any_sync(0xffffffffu, *(volatile const u32*)gt.p != 0);
 }
 
 // Whether this block is the last of n to come here (p[2] of the gate counts

@@ -467,6 +467,7 @@ __global__ void __launch_bounds__(128, 4)
 __global__ void __launch_bounds__(128) k_flow_links(FullLinks<double> U, Geom g, MatFix w, FixGate gt) {
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     u32 st = 0;
+    if (gate_lost(gt)) return;
     if (s < g.V) {
         const int mu = (int)blockIdx.y;
         const M3<double> u = U.load(s, mu);

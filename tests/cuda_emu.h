@@ -233,6 +233,8 @@ T __shfl_down_sync(unsigned, T v, int off) {
     return emu::shfl_down(v, off);
 }
 inline unsigned __ballot_sync(unsigned, int p) { return emu::ballot(p != 0); }
+inline int __any_sync(unsigned, int p) { return emu::ballot(p != 0) != 0; }
+inline int __all_sync(unsigned, int p) { return emu::ballot(p != 0) == ~0u; }
 inline unsigned __reduce_add_sync(unsigned, unsigned v) {
     for (int o = 16; o > 0; o >>= 1) v += emu::shfl_down(v, o);
     return v;

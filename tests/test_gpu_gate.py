@@ -1,5 +1,7 @@
 """complex128 calls around the gate between fixed point and FP64 (csrc/fix.cuh):
 fields and regions that have to stay in FP64, and what a shut gate costs."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -9,7 +11,7 @@ from flue_gb300 import _lib, generate
 from flue_gb300 import gluonCalc as G
 from flue_gb300.ensemble import Ensemble
 from flue_gb300.field import GaugeField, as_field
-from tests.test_gpu_fix import ALL, B2, _both, _flow_both
+from tests.test_gpu_fix import ALL, B2, _a, _both, _flow_both, _fp64_only_bytes, _ptr
 
 pytestmark = pytest.mark.gpu
 
@@ -83,3 +85,62 @@ def test_wmunu_table_adds_its_loops_exactly(seed):
         return G.wmunu_table(f, 2, 1, 4, 4)
 
     assert np.array_equal(table(64, 32), table(4, 4))
+
+
+def _shut_calls(f):
+    """name -> (call, full workspace, workspace of the FP64 kernels alone)."""
+    L, d, st = _lib.load(), f.descriptor(), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    v, nt = f.volume, f.nt
+    out = torch.empty(64, dtype=torch.float64, device="cuda")
+    field = torch.empty(9 * v, dtype=torch.complex128, device="cuda")
+    red = 1024  # partial sums at most
+
+    def ws(op):
+        return L.flue_workspace_bytes(op, *f.dims, _lib.C128)
+
+    return {
+        "plaquette": (lambda w, n: _lib.call("flue_plaquette", ctypes.byref(d), 1, 4, 4, _ptr(out), _ptr(w), n, st),
+                      ws(_lib.OP_PLAQUETTE), _a(min(red, (v + 255) // 256) * 8)),
+        "polyakov": (lambda w, n: _lib.call("flue_polyakov", ctypes.byref(d), _ptr(out), _ptr(w), n, st),
+                     ws(_lib.OP_POLYAKOV), _a(min(red, (v // nt + 7) // 8) * 16)),
+        "wmunu_table": (lambda w, n: _lib.call("flue_wmunu_table", ctypes.byref(d), 2, 1, 8, 8, _ptr(out), _ptr(w), n, st),
+                        L.flue_wmunu_table_bytes(*f.dims, _lib.C128, 8, 8), _a(16 * v * 144) + _a(64 * ((v + 127) // 128) * 8)),
+        "clover": (lambda w, n: _lib.call("flue_fmunu", ctypes.byref(d), _lib.FMUNU_CLOVER, 2, 1, _ptr(field), _ptr(w), n, st),
+                   ws(_lib.OP_FMUNU), _fp64_only_bytes(f.dims, 1, 2, False)),
+    }
+
+
+def _shut_field(dims, change):
+    f = GaugeField.empty(dims, "c128")
+    if change == "near_one":
+        f.storage.normal_().mul_(1e-4)
+        for a in range(3):
+            f.storage[a, a] += 1
+        f.reunitarise_()
+    else:
+        f.storage.normal_()
+        f.reunitarise_()
+        f.storage.mul_(1.01)
+    return f
+
+
+# Where FP64 has the field in the end, the fixed-point kernels in front of it have
+# to notice early: a few launches (20 us) and 5% of the FP64 time at most.
+@pytest.mark.parametrize("change", ["near_one", "not_unitary"])
+@pytest.mark.parametrize("call", ["plaquette", "polyakov", "wmunu_table", "clover"])
+def test_a_shut_gate_costs_little(call, change):
+    f = _shut_field((64, 32, 32, 32) if call == "polyakov" else (48, 24, 24, 24), change)
+    run, full, small = _shut_calls(f)[call]
+    assert full > small
+    w = torch.empty(full, dtype=torch.uint8, device="cuda")
+    times = {full: [], small: []}
+    for _ in range(12):
+        for n in times:
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            run(w, n)
+            b.record()
+            torch.cuda.synchronize()
+            times[n].append(a.elapsed_time(b) * 1e3)
+    t, t64 = np.median(times[full][3:]), np.median(times[small][3:])
+    assert t <= 1.05 * t64 + 20, (t, t64)

@@ -226,8 +226,9 @@ __device__ __forceinline__ void ff_addprod(FF& s, float a, float b) {
 // The same for sums that stay within +-2, in 4 instructions a product instead of
 // 10: hi carries 6 + the sum, so it keeps one exponent, every step of it is a
 // multiple of 2^-21 and known exactly, and what the step rounded off the product
-// (below 2^-22) goes to lo.  The sum is good to about 2^-43, far below the one
-// rounding of the result.  54 products a link: RK3 step at 32^3x64 2.94 -> 2.76 ms.
+// (below 2^-22) goes to lo.  The sum is good to about 2^-46 (2^-43 at worst), far
+// below the one rounding of the result, where that is not much smaller than 1
+// (reunitarise).  54 products a link: RK3 step at 32^3x64 2.94 -> 2.76 ms.
 struct FB {
     float hi, lo;
     __device__ __forceinline__ float sum() const { return __fadd_rn(__fsub_rn(hi, 6.0f), lo); }
@@ -333,7 +334,13 @@ __device__ __forceinline__ void reunitarise(M3<W>& w) {
     };
     rows();
     if constexpr (sizeof(W) == 4) {
-        if (!fix_su3_rows_f32<SumFB>(r, im)) {  // far from SU(3): sums of any size
+        // Off-diagonal entries that are small need sums exact to 2^-48 of
+        // themselves: near a diagonal matrix the general sums (as when a row is far
+        // from length 1).  At 2^-14 the bounded sums' 2^-46 is 2^-15 of the rounding.
+        float off = 0.f;
+#pragma unroll
+        for (int k : {1, 2, 3, 5}) off = fmaf(w.r[k], w.r[k], fmaf(w.i[k], w.i[k], off));
+        if (!(off > 0x1p-14f) || !fix_su3_rows_f32<SumFB>(r, im)) {
             rows();
             fix_su3_rows_f32<SumFF>(r, im);
         }

@@ -286,3 +286,9 @@ inline double __longlong_as_double(long long b) {
     memcpy(&x, &b, 8);
     return x;
 }
+inline float __fmul_rn(float a, float b) { return a * b; }
+inline float __fadd_rn(float a, float b) { return a + b; }
+inline float __fsub_rn(float a, float b) { return a - b; }
+inline float __fmaf_rn(float a, float b, float c) { return fmaf(a, b, c); }
+inline float emu_rsqrtf(float x) { return 1.0f / sqrtf(x); }
+#define rsqrtf emu_rsqrtf

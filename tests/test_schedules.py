@@ -43,7 +43,7 @@ def _build(tmp_path, body):
     (tmp_path / "main.cpp").write_text('#include "cuda_emu.h"\n#include "fix.cuh"\n#include "loop5.cuh"\n'
                                        '#include "loop5_fix.cuh"\nnamespace flue {\n' + body)
     exe = tmp_path / "main"
-    r = subprocess.run([shutil.which("g++"), "-std=c++17", "-O1", "-w", "-pthread", "-I", str(tmp_path), "-I", HERE, "-I",
+    r = subprocess.run([shutil.which("g++"), "-std=c++17", "-O1", "-ffp-contract=off", "-w", "-pthread", "-I", str(tmp_path), "-I", HERE, "-I",
                         include, str(tmp_path / "main.cpp"), "-o", str(exe)], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr[-4000:]
     return str(exe)

@@ -749,10 +749,21 @@ static bool cpu_writable(const void* p) {
 // pages, and a GPU fault each costs far more than the write: a gradient of
 // 24^3x48 complex128 (382 MB, 64 KB pages) took 98 ms of faults, one thread
 // maps it in 13 ms; the call with a fresh gradient takes 17.0 ms with one thread,
-// 12.9 with 2, 11.4 with 4, 13.4 with 8.  Runs beside the first
+// 12.9 with 2, 11.4 with 4, 13.4 with 8.  Runs beside the first slab's
 // kernels (FLUE_MAP_THREADS); wait() before the first one that writes the array.
+// An array that has its pages is left alone: four of them are looked at, spread
+// over it (1.5 us each; the threads and their walk over the pages made an 8^3x16
+// call 0.14 -> 0.20 ms and a 24^3x48 one 4.2 -> 5.6).
 class PageMapper {
     std::vector<std::thread> th_;
+    static bool mapped(uintptr_t lo, uintptr_t hi, uintptr_t page) {
+        const uintptr_t last = (hi - 1 - lo) / page;
+        for (uintptr_t k = 0; k < 4; ++k) {
+            unsigned char in = 0;
+            if (mincore((void*)(lo + last * k / 3 * page), page, &in) != 0 || !(in & 1)) return false;
+        }
+        return true;
+    }
     static void map(uintptr_t lo, uintptr_t hi) {
         if (lo < hi) (void)madvise((void*)lo, hi - lo, 23 /* MADV_POPULATE_WRITE */);
     }
@@ -767,6 +778,7 @@ class PageMapper {
         }
         if (a.type != cudaMemoryTypeUnregistered) return;
         const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), lo = (uintptr_t)p & ~(page - 1), hi = (uintptr_t)p + n;
+        if (mapped(lo, hi, page)) return;
         const size_t most = (size_t)std::max(1, env_int("FLUE_MAP_THREADS", 4));
         const size_t nt = std::min(most, std::max<size_t>(1, n >> 22));  // 4 MB a thread at least
         const uintptr_t per = ((hi - lo) / nt + page) & ~(page - 1);

@@ -123,7 +123,10 @@ cudaError_t launch_energy_slab_out(const FieldRef& U, const PlaneSet& ps, int64_
 // launch_energy over nslab time slabs on nstream (<= 4) streams forked from
 // st (plane sets without the time direction); workspace of
 // energy_slabs_ws_bytes(...) bytes.  Results equal launch_energy's: the
-// gradient bitwise, the energy up to the order of the FP64 partial sums.
+// gradient bitwise, the energy up to the order of the FP64 partial sums.  A
+// complex128 slab has a gate of its own (fix.cuh): where some slabs of a field
+// take fixed point and others FP64, the two calls differ by the rounding of the
+// ones that one pass decides the other way.
 size_t energy_slabs_ws_bytes(const Geom& g, int prec, const PlaneSet& ps, bool with_force, int nslab, int nstream);
 size_t energy_slabs_ws_min_bytes(const Geom& g, int prec, const PlaneSet& ps, bool with_force, int nslab, int nstream);
 cudaError_t launch_energy_slabs(const FieldRef& U, const PlaneSet& ps, double* out_E, void* force, int form, void* ws,

@@ -7,7 +7,7 @@ import pytest
 
 torch = pytest.importorskip("torch")
 
-from flue_gb300 import _lib, generate
+from flue_gb300 import _lib, forces, generate
 from flue_gb300 import gluonCalc as G
 from flue_gb300.ensemble import Ensemble
 from flue_gb300.field import GaugeField, as_field
@@ -144,3 +144,26 @@ def test_a_shut_gate_costs_little(call, change):
             times[n].append(a.elapsed_time(b) * 1e3)
     t, t64 = np.median(times[full][3:]), np.median(times[small][3:])
     assert t <= 1.05 * t64 + 20, (t, t64)
+
+
+# One link that is not unitary: in one pass the whole field is in FP64, in slabs
+# the slab with that link.  Slabs that decide as one pass does give its gradient bit
+# for bit, the others to the rounding of test_gpu_fix (8e-15 of its norm).
+def test_each_time_slab_has_its_own_gate(monkeypatch):
+    u = np.array(generate.random_field((8, 6, 5, 4), 0.3, 9))
+    u[3, 2, 1, 0, 2] *= 1.01
+    f = as_field(np.asfortranarray(u))
+
+    def run(slabs):
+        monkeypatch.setenv("FLUE_SLABS", str(slabs))
+        e, g = forces.magnetic_force(f)
+        return e, g.cpu().numpy()
+
+    (e1, g1), (e4, g4) = run(1), run(4)
+    assert np.array_equal(g4[2:4], g1[2:4])
+    for t in (0, 4, 6):
+        assert not np.array_equal(g4[t:t + 2], g1[t:t + 2])
+    assert np.linalg.norm(g4 - g1) <= 8e-15 * np.linalg.norm(g1) and abs(e4 - e1) <= 1e-14 * abs(e1)
+    u[..., 1:, :, :] *= 1.01  # no slab in fixed point
+    f = as_field(np.asfortranarray(u))
+    assert np.array_equal(run(4)[1], run(1)[1])

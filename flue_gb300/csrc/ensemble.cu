@@ -257,7 +257,8 @@ __global__ void __launch_bounds__(BS, (FlowMinBlocks<T, BS>::value)) k_ens_flow(
             const EnsField f = a.fields[sl.field];
             const Geom g = make_geom(sl.nts, f.g.n[1], f.g.n[2], f.g.n[3]);
             using VP = decltype(MatAoS<T>::p);
-            const MatAoS<T> lines{reinterpret_cast<VP>(a.ring + (size_t)(j % kSlots) * a.slot_bytes), g.V};
+            const MatAoS<T> lines{reinterpret_cast<VP>(a.ring + (size_t)(j % kSlots) * a.slot_bytes), g.V,
+                                  3 * a.pa.nd};
             const int64_t s = (int64_t)tk.b * BS + threadIdx.x;
             if (tk.type == TASK_LINES) {
                 // the slot is free once every FWD task of its last slab is done
@@ -392,7 +393,8 @@ __global__ void __launch_bounds__(3 * EF_BS) k_ens_flow_fix(EnsFlowArgs a) {
             const int j = tk.a;
             const EnsSlab sl = a.slabs[j];
             const Geom g = make_geom(sl.nts, f.g.n[1], f.g.n[2], f.g.n[3]);
-            const MatFix lines{(int4*)(a.ring + (size_t)(j % kSlots) * a.slot_bytes), g.V};
+            const MatFix lines{(int4*)(a.ring + (size_t)(j % kSlots) * a.slot_bytes), g.V,
+                                  3 * a.pa.nd};
             if (tk.type == TASK_LINES) {
                 if (threadIdx.x < 32) {
                     const int i = ring_prev(a, j, true, mixed);

@@ -703,8 +703,8 @@ __global__ void __launch_bounds__(3 * FF_BS, FF_MINB)
 template <typename I>
 static void flow_fix_stages(void* links, const Geom& g, double eps, char* ws, const FlowFixWs& w, const FixGate& gt,
                             cudaStream_t st) {
-    const MatFix w0{(int4*)ws, g.V}, w1{(int4*)(ws + w.w1), g.V};
-    const AHFix xb{(longlong2*)(ws + w.x), g.V};
+    const MatFix w0{(int4*)ws, g.V, 4}, w1{(int4*)(ws + w.w1), g.V, 4};
+    const AHFix xb{(longlong2*)(ws + w.x), g.V, 4};
     const unsigned nb = (unsigned)((g.V + FF_BS - 1) / FF_BS) * 4;
     // Z = -eps TA(U N): the kernel holds (U N - (U N)^+)/64 off the diagonal and
     // (3 Im - trace)/64 on it.  The kept X of stage 0 is Z0/4, so stage 1 takes
@@ -760,7 +760,7 @@ cudaError_t launch_wflow_step(void* links, const Geom& g, int prec, double eps, 
         gt.need = (u32)g.V;  // a quarter of the links
         cudaError_t e = cudaMemsetAsync(gt.p, 0, GATE_WORDS * sizeof(u32), st);
         if (e != cudaSuccess) return e;
-        const MatFix w0{(int4*)w, g.V};
+        const MatFix w0{(int4*)w, g.V, 4};
         note_launch(), k_flow_links<<<dim3((unsigned)((g.V + 127) / 128), 4), 128, 0, st>>>(
             FullLinks<double>{(const double2*)links, g.V}, g, w0, gt);
         if (MatFix::fits32(g.V, 4))

@@ -958,9 +958,9 @@ template <class L, typename T>
 static cudaError_t energy_fwd_part(const L& U, const Geom& g, const Geom& gs, int t0, const PlaneArg& pa, int kind,
                                    double* out_E, bool with_force, double vnorm, char* ws, const EnergyWs& w,
                                    RefOut<T> fout, cudaStream_t st) {
-    MatAoS<T> lines{reinterpret_cast<decltype(MatAoS<T>::p)>(ws + w.lines), g.V};
-    AHAoS<T> kb{with_force ? reinterpret_cast<decltype(AHAoS<T>::p)>(ws + w.kbuf) : nullptr, g.V};
-    MatAoS<T> lam{reinterpret_cast<decltype(MatAoS<T>::p)>(ws + w.lam), g.V};
+    MatAoS<T> lines{reinterpret_cast<decltype(MatAoS<T>::p)>(ws + w.lines), g.V, 3 * pa.nd};
+    AHAoS<T> kb{with_force ? reinterpret_cast<decltype(AHAoS<T>::p)>(ws + w.kbuf) : nullptr, g.V, pa.np};
+    MatAoS<T> lam{reinterpret_cast<decltype(MatAoS<T>::p)>(ws + w.lam), g.V, 3 * pa.nd};
     double* part = out_E ? (double*)(ws + w.part) : nullptr;
     const unsigned nbl = (unsigned)((g.V + 127) / 128);
     const int fbs = w.fix ? fix_fwd_block(g.V, pa.np) : FWD_BS;  // sites a block of the forward covers
@@ -973,8 +973,8 @@ static cudaError_t energy_fwd_part(const L& U, const Geom& g, const Geom& gs, in
     stage_mark(0, st);
     if constexpr (sizeof(T) == 8) {
         const FixGate gt = energy_gate(g, pa, ws, w);
-        const MatFix flines{(int4*)(ws + w.lines), g.V};
-        const AHFix fkb{with_force ? (longlong2*)(ws + w.kbuf) : nullptr, g.V};
+        const MatFix flines{(int4*)(ws + w.lines), g.V, 3 * pa.nd};
+        const AHFix fkb{with_force ? (longlong2*)(ws + w.kbuf) : nullptr, g.V, pa.np};
         const bool ffits = MatFix::fits32(g.V, 3 * pa.nd);
         if (w.fix) {
             if ((e = cudaMemsetAsync(gt.p, 0, w.gate_bytes, st)) != cudaSuccess) return e;
@@ -1031,8 +1031,8 @@ static cudaError_t energy_fwd_part(const L& U, const Geom& g, const Geom& gs, in
     if (!with_force) return cudaSuccess;
     if constexpr (sizeof(T) == 8) {
         const FixGate gt = energy_gate(g, pa, ws, w);
-        const MatFix flines{(int4*)(ws + w.lines), g.V}, flam{(int4*)(ws + w.lam), g.V};
-        const AHFix fkb{(longlong2*)(ws + w.kbuf), g.V};
+        const MatFix flines{(int4*)(ws + w.lines), g.V, 3 * pa.nd}, flam{(int4*)(ws + w.lam), g.V, 3 * pa.nd};
+        const AHFix fkb{(longlong2*)(ws + w.kbuf), g.V, pa.np};
         const unsigned nl = nbc * 3 * pa.nd, gl = gated_grid(w, nl);
         if (w.fix) {
             const unsigned nlf = (unsigned)((g.V + FIX_BS - 1) / FIX_BS) * 3 * pa.nd;
@@ -1063,8 +1063,8 @@ template <typename T>
 static cudaError_t energy_out_part(const Geom& g, const PlaneArg& pa, double vnorm, int form, char* ws,
                                    const EnergyWs& w, RefOut<T> fo, unsigned max_blocks, cudaStream_t st,
                                    bool skip_zero = false) {
-    MatAoS<T> lines{reinterpret_cast<decltype(MatAoS<T>::p)>(ws + w.lines), g.V};
-    MatAoS<T> lam{reinterpret_cast<decltype(MatAoS<T>::p)>(ws + w.lam), g.V};
+    MatAoS<T> lines{reinterpret_cast<decltype(MatAoS<T>::p)>(ws + w.lines), g.V, 3 * pa.nd};
+    MatAoS<T> lam{reinterpret_cast<decltype(MatAoS<T>::p)>(ws + w.lam), g.V, 3 * pa.nd};
     const T scale = (T)(-1.0 / (2.0 * vnorm));
     unsigned nb = (unsigned)((g.V + 127) / 128);
     if (max_blocks && nb > max_blocks) nb = max_blocks;
@@ -1073,7 +1073,7 @@ static cudaError_t energy_out_part(const Geom& g, const PlaneArg& pa, double vno
     if constexpr (sizeof(T) == 8) {
         gt = energy_gate(g, pa, ws, w);
         if (w.fix) {
-            const MatFix flines{(int4*)(ws + w.lines), g.V}, flam{(int4*)(ws + w.lam), g.V};
+            const MatFix flines{(int4*)(ws + w.lines), g.V, 3 * pa.nd}, flam{(int4*)(ws + w.lam), g.V, 3 * pa.nd};
             note_launch(), k_linkcot_fix<<<dim3(nb, 4), 128, 0, st>>>(g, pa, flines, flam, scale, form, fo, skip_zero,
                                                                    gt.p + GATE_WORDS, pa.slot[0] < 0, gt);
             nbg = gated_grid(w, nb);

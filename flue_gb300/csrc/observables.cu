@@ -946,8 +946,8 @@ cudaError_t launch_wmunu_table(const FieldRef& U, int mu, int nu, int rmax, int 
         cudaError_t e;
         const FixGate gt = red_gate(ws, fws, 0, st, &e);
         if (e != cudaSuccess) return e;
-        const MatFix fl{(int4*)ws, g.V};
-        const MatAoS<double> dl{(double2*)ws, g.V};
+        const MatFix fl{(int4*)ws, g.V, rmax + tmax};
+        const MatAoS<double> dl{(double2*)ws, g.V, rmax + tmax};
         const unsigned cap = 8u * (unsigned)device_sms(), nsf = (unsigned)((g.V + WTF_BS - 1) / WTF_BS);
         note_launch(), k_wt_lines_fix<<<dim3(nsb, 2), WT_BS, 0, st>>>(L, g, mu, nu, rmax, tmax, fl, gt);
         i64* ipart = reinterpret_cast<i64*>(part);
@@ -962,7 +962,7 @@ cudaError_t launch_wmunu_table(const FieldRef& U, int mu, int nu, int rmax, int 
         return cudaGetLastError();
     }
     FLUE_DISPATCH_LINKS(U, {
-        MatAoS<T> ln{reinterpret_cast<decltype(MatAoS<T>::p)>(ws), g.V};
+        MatAoS<T> ln{reinterpret_cast<decltype(MatAoS<T>::p)>(ws), g.V, rmax + tmax};
         note_launch(), k_wt_lines<decltype(L), T><<<nsb, WT_BS, 0, st>>>(L, g, mu, nu, rmax, tmax, ln);
         note_launch(), k_wt_loops<T><<<nsb * nrt, WT_BS, 0, st>>>(g, mu, nu, rmax, tmax, ln, part);
     });

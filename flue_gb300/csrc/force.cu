@@ -1295,12 +1295,15 @@ cudaError_t launch_fmunu(const FieldRef& U, int kind, int mu, int nu, void* out,
     if (kind == 0 && U.prec != PREC_C128) {
         const RefOut<float> fo{(float2*)out, U.g.V, 1};
         const unsigned nb = (unsigned)((U.g.V + FWD_BS - 1) / FWD_BS);
+        stage_mark(0, st);
+        stage_mark(1, st);  // (no lines)
         if (U.prec == PREC_R12)
             note_launch(), k_clover<R12Links, int64_t><<<nb, FWD_BS, 0, st>>>(R12Links{(const float4*)U.links, U.g.V}, U.g, mu, nu, fo);
         else if (FullLinks32::fits(U.g.V))
             note_launch(), k_clover<FullLinks32, u32><<<nb, FWD_BS, 0, st>>>(FullLinks32{(const char*)U.links, (u32)U.g.V}, U.g, mu, nu, fo);
         else
             note_launch(), k_clover<FullLinks<float>, int64_t><<<nb, FWD_BS, 0, st>>>(FullLinks<float>{(const float2*)U.links, U.g.V}, U.g, mu, nu, fo);
+        stage_mark(2, st);
         return cudaGetLastError();
     }
     FLUE_DISPATCH_LINKS(U, {

@@ -33,15 +33,18 @@ size_t wflow_ws_min_bytes(const Geom& g) {
     return ((f + 255) & ~(size_t)255) + ((b + 255) & ~(size_t)255) + ((p + 255) & ~(size_t)255);
 }
 
-// the fixed-point step's scratch: two link fields, X of the last stage, the
-// gate (the FP64 step's buffers, used when the gate is shut, lie over the
-// fields)
+// the fixed-point step's scratch: a link field, X of the last stage, the gate
+// (the FP64 step's buffers, used when the gate is shut, lie over the first two).
+// The other link field of the stages is the caller's own: a converted link has the
+// size of a complex128 one, and whole tiles of 32 sites fill it exactly; other
+// lattices take a second one here (w1 > 0).  So the step needs no more memory
+// than in FP64.
 struct FlowFixWs {
     size_t w1, x, gate, total;
 };
 static FlowFixWs flow_fix_layout(const Geom& g) {
     FlowFixWs w;
-    w.w1 = MatFix::bytes(g.V, 4);
+    w.w1 = g.V % 32 ? MatFix::bytes(g.V, 4) : 0;
     w.x = w.w1 + MatFix::bytes(g.V, 4);
     w.gate = std::max(w.x + AHFix::bytes(g.V, 4), wflow_ws_min_bytes(g));
     w.total = w.gate + 256;
@@ -463,8 +466,8 @@ __global__ void __launch_bounds__(128, 4)
 // ---------------------------------------------------------------------------
 // The step of a complex128 field in fixed point (fix.cuh): the links are
 // converted once (k_flow_links), each stage computes the force of a link and
-// moves it in one kernel from one fixed-point field to the other, and the last
-// stage writes the complex128 links.  A thread carries one column of a link
+// moves it in one kernel from one fixed-point field to the other (the second lies
+// over the complex128 links, FlowFixWs), and the last stage writes those.  A thread carries one column of a link
 // (three warps for 32 sites), as the 5-loop kernels do.  A stage is 13 matrix
 // products and exp(X) a link, bound by the integer multiply-add pipe.  RK3 step
 // at 32^3x64: 92.8 ms as FP64 force and update, 22.2 with exp(X) from its even
@@ -703,7 +706,7 @@ __global__ void __launch_bounds__(3 * FF_BS, FF_MINB)
 template <typename I>
 static void flow_fix_stages(void* links, const Geom& g, double eps, char* ws, const FlowFixWs& w, const FixGate& gt,
                             cudaStream_t st) {
-    const MatFix w0{(int4*)ws, g.V, 4}, w1{(int4*)(ws + w.w1), g.V, 4};
+    const MatFix w0{(int4*)ws, g.V, 4}, w1{(int4*)(w.w1 ? ws + w.w1 : links), g.V, 4};
     const AHFix xb{(longlong2*)(ws + w.x), g.V, 4};
     const unsigned nb = (unsigned)((g.V + FF_BS - 1) / FF_BS) * 4;
     // Z = -eps TA(U N): the kernel holds (U N - (U N)^+)/64 off the diagonal and

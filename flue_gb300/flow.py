@@ -12,12 +12,17 @@ import os
 import torch
 
 from . import _lib, gluonCalc
-from .field import GaugeField, _ptr, _stream_handle, as_field, workspace
+from .field import GaugeField, Workspace, _ptr, _stream_handle, as_field, workspace
 
 
 def wflow_step(field: GaugeField, eps: float) -> GaugeField:
     """One RK3 step in place (c128 or c64 field)."""
-    ws = workspace(_lib.OP_WFLOW, field)
+    try:
+        ws = workspace(_lib.OP_WFLOW, field)
+    except torch.cuda.OutOfMemoryError:
+        # the FP64 step's scratch, as large as that of a complex64 field: less than
+        # a c128 field asks for when its sites are not a multiple of 32
+        ws = Workspace.get(_lib.load().flue_workspace_bytes(_lib.OP_WFLOW, *field.dims, _lib.C64), field.device)
     d = field.descriptor()
     with torch.cuda.device(field.device):
         _lib.call("flue_wflow_step", ctypes.byref(d), float(eps), _ptr(ws), ws.numel(), _stream_handle())

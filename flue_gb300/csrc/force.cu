@@ -131,11 +131,11 @@ static PatchArg make_patch(const Geom& g, const PlaneArg& pa, int bs) {
 //    for a whole lattice; a time slab of a larger field otherwise -- the lines
 //    never step in time then).
 // ---------------------------------------------------------------------------
-template <class L, typename T>
-__global__ void k_lines(L U, Geom g, Geom gs, int t0, PlaneArg pa, MatAoS<T> lines) {
+template <class L>
+__global__ void k_lines(L U, Geom g, Geom gs, int t0, PlaneArg pa, MatAoS<float> lines) {
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= g.V) return;
-    line_site<L, T>(U, g, gs, t0, pa, lines, s, (int)blockIdx.y);
+    line_site<L, float>(U, g, gs, t0, pa, lines, s, (int)blockIdx.y);
 }
 
 // complex128 fields: the lines in fixed point (fix.cuh), counting the links
@@ -175,8 +175,10 @@ __global__ void __launch_bounds__(128) k_lines_gated(FullLinks<double> U, Geom g
 // ---------------------------------------------------------------------------
 // 2. forward: one thread per (site, plane)
 // ---------------------------------------------------------------------------
-// block size and minimum resident blocks per SM (register budget) of the
-// forward and line-cotangent kernels; overridable at build time
+// block size and, in FP32, minimum resident blocks per SM (register budget) of
+// the forward and line-cotangent kernels; overridable at build time.  The FP64
+// kernels keep every register they need (they are bound by the FP64 pipe, not by
+// latency).
 #ifndef FLUE_FWD_BS
 #define FLUE_FWD_BS 128
 #endif
@@ -194,16 +196,6 @@ __global__ void __launch_bounds__(128) k_lines_gated(FullLinks<double> U, Geom g
 #ifndef FLUE_COT_MINB
 #define FLUE_COT_MINB 4
 #endif
-// the register caps apply to the FP32 kernels; the FP64 ones keep every
-// register they need (they are bound by the FP64 pipe, not by latency)
-template <typename T>
-struct MinBlocks {
-    static constexpr int fwd = 1, cot = 1;
-};
-template <>
-struct MinBlocks<float> {
-    static constexpr int fwd = FLUE_FWD_MINB, cot = FLUE_COT_MINB;
-};
 constexpr int FWD_BS = FLUE_FWD_BS;
 // Sites a block of the fixed-point forward and line cotangents covers, three
 // threads a site: 192 threads and up to 168 registers, two blocks an SM.  Both
@@ -253,11 +245,12 @@ __device__ __forceinline__ void fwd_block(unsigned b, const Geom& g, const Plane
     }
 }
 
-template <typename T, typename I>
-__global__ void __launch_bounds__(FWD_BS, MinBlocks<T>::fwd)
-    k_fwd(Geom g, PlaneArg pa, int kind, PatchArg pt, MatAoS<T> lines, AHAoS<T> kout, RefOut<T> fout, double* part) {
+template <typename I>
+__global__ void __launch_bounds__(FWD_BS, FLUE_FWD_MINB)
+    k_fwd(Geom g, PlaneArg pa, int kind, PatchArg pt, MatAoS<float> lines, AHAoS<float> kout, RefOut<float> fout,
+          double* part) {
     __shared__ double sh[32];
-    fwd_block<T, I>(blockIdx.x, g, pa, kind, pt, lines, kout, fout, part, sh);
+    fwd_block<float, I>(blockIdx.x, g, pa, kind, pt, lines, kout, fout, part, sh);
 }
 
 template <typename I>
@@ -594,10 +587,10 @@ __device__ __forceinline__ void linecot_block(unsigned b, const Geom& g, const P
     lam.store(s64, 3 * slot + len - 1, acc);
 }
 
-template <typename T, typename I>
-__global__ void __launch_bounds__(COT_BS, MinBlocks<T>::cot)
-    k_linecot(Geom g, PlaneArg pa, MatAoS<T> lines, AHAoS<T> kin, MatAoS<T> lam) {
-    linecot_block<T, I>(blockIdx.x, g, pa, lines, kin, lam);
+template <typename I>
+__global__ void __launch_bounds__(COT_BS, FLUE_COT_MINB)
+    k_linecot(Geom g, PlaneArg pa, MatAoS<float> lines, AHAoS<float> kin, MatAoS<float> lam) {
+    linecot_block<float, I>(blockIdx.x, g, pa, lines, kin, lam);
 }
 
 template <typename I>
@@ -1004,7 +997,7 @@ static cudaError_t energy_fwd_part(const L& U, const Geom& g, const Geom& gs, in
         else
             fwd64(k_fwd_gated<int64_t>);
     } else {
-        note_launch(), k_lines<L, T><<<dim3(nbl, pa.nd), 128, 0, st>>>(U, g, gs, t0, pa, lines);
+        note_launch(), k_lines<L><<<dim3(nbl, pa.nd), 128, 0, st>>>(U, g, gs, t0, pa, lines);
         stage_mark(1, st);
         bool tiled = false;
         if (fwd_tile_ok(g, pa, kind, fout.p != nullptr, fits)) {
@@ -1017,9 +1010,9 @@ static cudaError_t energy_fwd_part(const L& U, const Geom& g, const Geom& gs, in
         }
         if (!tiled) {
             if (fits)
-                note_launch(), k_fwd<T, uint32_t><<<nbx * pa.np, FWD_BS, 0, st>>>(g, pa, kind, pt, lines, kb, fout, part);
+                note_launch(), k_fwd<uint32_t><<<nbx * pa.np, FWD_BS, 0, st>>>(g, pa, kind, pt, lines, kb, fout, part);
             else
-                note_launch(), k_fwd<T, int64_t><<<nbx * pa.np, FWD_BS, 0, st>>>(g, pa, kind, pt, lines, kb, fout, part);
+                note_launch(), k_fwd<int64_t><<<nbx * pa.np, FWD_BS, 0, st>>>(g, pa, kind, pt, lines, kb, fout, part);
         }
     }
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -1050,9 +1043,9 @@ static cudaError_t energy_fwd_part(const L& U, const Geom& g, const Geom& gs, in
             note_launch(), k_linecot_gated<int64_t><<<gl, COT_BS, 0, st>>>(g, pa, lines, kb, lam, nl, gt);
     } else {
         if (cfits)
-            note_launch(), k_linecot<T, uint32_t><<<nbc * 3 * pa.nd, COT_BS, 0, st>>>(g, pa, lines, kb, lam);
+            note_launch(), k_linecot<uint32_t><<<nbc * 3 * pa.nd, COT_BS, 0, st>>>(g, pa, lines, kb, lam);
         else
-            note_launch(), k_linecot<T, int64_t><<<nbc * 3 * pa.nd, COT_BS, 0, st>>>(g, pa, lines, kb, lam);
+            note_launch(), k_linecot<int64_t><<<nbc * 3 * pa.nd, COT_BS, 0, st>>>(g, pa, lines, kb, lam);
     }
     stage_mark(3, st);
     return cudaGetLastError();

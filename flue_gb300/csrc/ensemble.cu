@@ -119,8 +119,11 @@ __device__ __forceinline__ int ring_prev(const EnsFlowArgs& a, int j, bool open,
 }
 
 // Counts every field's links in its gate (all four directions: a quarter of
-// them has to be away from 1).  Fields too long for the Polyakov product's
-// bounds count as not unitary.
+// them has to be away from 1).  B^2 only knows the spatial links and the Polyakov
+// loop the others, so either may be small while the rest of the field is rough: a
+// near_patch of spatial links, or 32 time links in a row that are close to 1 but not
+// all equal to it (temporal gauge), shut the gate.  Fields too long for the Polyakov
+// product's bounds count as not unitary.
 __global__ void __launch_bounds__(128) k_ens_gates(EnsFlowArgs a) {
     for (int f = blockIdx.y; f < a.nfields; f += gridDim.y) {
         const EnsField fl = a.fields[f];
@@ -132,10 +135,20 @@ __global__ void __launch_bounds__(128) k_ens_gates(EnsFlowArgs a) {
             const int64_t i = i0 + threadIdx.x;
             u32 st = 0;
             if (gate_lost(gt)) break;
+            const int mu = (i >= fl.g.V) + (i >= 2 * fl.g.V) + (i >= 3 * fl.g.V);
+            M3<double> u = m_zero<double>();
             if (i < n) {
-                const M3<double> u = U.load(i % fl.g.V, (int)(i / fl.g.V));
+                const int64_t s = i - (int64_t)mu * fl.g.V;
+                u = U.load(s, mu);
                 st = link_state(u, fx_of(u));
+                if (st == 0 && mu > 0) {
+                    int c[4];
+                    site_coords(fl.g, s, c);
+                    for (int nu = mu + 1; nu < 4; ++nu)
+                        if (near_patch(U, fl.g, c, mu, nu)) st = 1;
+                }
             }
+            if (__all_sync(0xffffffffu, st == 0 && mu == 0) && !__all_sync(0xffffffffu, is_one(u))) st = 1;
             gate_count(gt, st);
         }
     }

@@ -422,6 +422,13 @@ __device__ __forceinline__ u32 link_state(const M3<double>& u, const M3F& f) {
     return (ok ? 0u : 1u) | (dist2_one(r, i) > FIX_FAR2 ? 2u : 0u);
 }
 
+__device__ __forceinline__ bool is_one(const M3<double>& u) {
+    bool one = true;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) one = one && u.r[k] == (k % 4 == 0 ? 1.0 : 0.0) && u.i[k] == 0.0;
+    return one;
+}
+
 // Whether the twelve links of the four plaquettes in the plane (d, e) around the
 // site at coordinates c are all close to 1.  For sites whose link along d is,
 // rare in a rough field; most calls end with the first link, the one along e.

@@ -167,3 +167,40 @@ def test_each_time_slab_has_its_own_gate(monkeypatch):
     u[..., 1:, :, :] *= 1.01  # no slab in fixed point
     f = as_field(np.asfortranarray(u))
     assert np.array_equal(run(4)[1], run(1)[1])
+
+
+# B^2 sees only the spatial links and the Polyakov loop only the others: either part
+# close to 1, the rest rough.  Both sides then run in FP64 and only add in another
+# order: sums of V squares, and of the columns' imaginary traces.
+@pytest.mark.parametrize("part", ["space", "time"])
+@pytest.mark.parametrize("dist", [1e-8, 1e-4])
+def test_ensemble_field_with_one_part_near_one(part, dist):
+    dims = (32, 5, 4, 3)
+    u, c = np.array(generate.haar_field(dims, 3)), np.array(generate.random_field(dims, dist, 4))
+    where = slice(1, 4) if part == "space" else slice(0, 1)
+    u[..., where, :, :] = c[..., where, :, :]
+    f = as_field(np.asfortranarray(u))
+    row = Ensemble([f]).run()[0]
+    if part == "space":
+        b2 = G.magnetic(f)
+        assert abs(row[4] - b2) <= 1e-14 * b2
+    else:
+        p = u[0, ..., 0, :, :]
+        for t in range(1, dims[0]):
+            p = p @ u[t, ..., 0, :, :]
+        scale = np.abs(np.trace(p, axis1=-2, axis2=-1).imag).sum()
+        assert abs(row[3] - G.polyakov(f, return_imag=True)[3]) <= 1e-14 * scale
+
+
+# (one sum in either arithmetic is often the same double: eight fields)
+def test_ensemble_in_temporal_gauge_takes_fixed_point():
+    fields = []
+    for seed in range(8):
+        u = np.array(generate.random_field((32, 4, 4, 4), 0.3, seed))
+        u[..., 0, :, :] = np.eye(3)
+        fields.append(as_field(np.asfortranarray(u)))
+        u[0, 0, 0, 0, 0] *= 1.01  # (no part in B^2)
+        fields.append(as_field(np.asfortranarray(u)))
+    b2 = Ensemble(fields).run()[:, 4].reshape(8, 2)
+    assert (b2[:, 0] != b2[:, 1]).any()
+    assert (np.abs(b2[:, 0] - b2[:, 1]) <= 1e-14 * b2[:, 1]).all()

@@ -338,11 +338,12 @@ __device__ __forceinline__ void reunitarise(M3<W>& w) {
     rows();
     if constexpr (sizeof(W) == 4) {
         // Off-diagonal entries that are small need sums exact to 2^-48 of
-        // themselves: near a diagonal matrix the general sums (as when a row is far
-        // from length 1).  At 2^-14 the bounded sums' 2^-46 is 2^-15 of the rounding.
+        // themselves: near a diagonal matrix (row 0 tells) the general sums, as when a
+        // row is far from length 1.  At 2^-14 the bounded sums' 2^-46 is 2^-15 of the
+        // rounding.
         float off = 0.f;
 #pragma unroll
-        for (int k : {1, 2, 3, 5}) off = fmaf(w.r[k], w.r[k], fmaf(w.i[k], w.i[k], off));
+        for (int k = 1; k < 3; ++k) off = fmaf(w.r[k], w.r[k], fmaf(w.i[k], w.i[k], off));
         if (!(off > 0x1p-14f) || !fix_su3_rows_f32<SumFB>(r, im)) {
             rows();
             fix_su3_rows_f32<SumFF>(r, im);

@@ -27,6 +27,7 @@
 #undef __constant__
 #undef __forceinline__
 #undef __launch_bounds__
+#undef __noinline__
 #define __shared__ static thread_local
 #define __global__ static
 #define __device__
@@ -34,6 +35,7 @@
 #define __constant__ const
 #define __forceinline__ inline
 #define __launch_bounds__(...)
+#define __noinline__
 
 namespace emu {
 

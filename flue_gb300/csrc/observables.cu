@@ -560,8 +560,8 @@ __global__ void __launch_bounds__(RED_BS) k_polyakov_finish(FullLinks<double> U,
 // The links are counted in the gate; k_polyakov_finish replaces the sums when it
 // turns out shut.  The imaginary part of the trace of a cold column is small, so a
 // quarter of the links has to be away from 1, and the first warp that finds none
-// among 32 ends the work of all, as does a link that is not unitary: a cold 32^3x64 took 1.13 ms when every block went on, 0.56 so,
-// 0.54 without fixed point.
+// among 32 ends the work of all, as does a link that is not unitary: a cold
+// 32^3x64 took 1.13 ms when every block went on, 0.56 so, 0.54 without fixed point.
 constexpr int POLF_BS = 128;
 static int polyfix_lanes(int nt) {
     int nl = 1;
